@@ -718,7 +718,12 @@ static int solve_phase(spk_plan *P, const int *rp, const int *ci, const void *ai
         o->relres_max = worst;
         o->sweeps = sweep;
         if (worst <= o->tol) return SPK_OK;
-        if (sweep >= o->max_refine) return SPK_ECONV;
+        if (sweep >= o->max_refine) { /* a kernel that gave up on a copy shows here: say so */
+            unsigned e[4];
+            TRY(spk_memcpy_d2h(e, P->d_err, sizeof e, stream));
+            TRY(spk_stream_sync(stream));
+            return e[0] & SPK_DEV_ERR_TIMEOUT ? SPK_ETIMEOUT : SPK_ECONV;
+        }
         TRY(spike_apply_once(P, x, r, nrhs, red, 1, stream));
     }
 }
