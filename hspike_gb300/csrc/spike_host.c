@@ -328,6 +328,26 @@ static int choose_partitions(int n, int KB, int requested)
     return (int)p;
 }
 
+/* A partition count the caller asked for may leave the GPU to a few long
+ * chains (the reference's p = 4 on a pentadiagonal n = 100,000: eight half
+ * chains of 6,250 dependent steps, 12.4 ms).  Each of the p partitions is then
+ * split into *sub pieces, as many as fill the GPU like an automatic count
+ * does while a piece keeps at least 16 tiles (8 from 64-row tiles on), so that
+ * both its halves are still eliminated at once; tiles up to 4 rows stop at the
+ * 2,048 partitions that are eliminated from both ends.  The p boundaries stay
+ * partition boundaries and p stays what spike_get_info reports.  With 512
+ * pieces each, the p = 4 solve takes 0.27 ms; 512 partitions of a complex
+ * heptadiagonal n = 4,000,000 in 4 pieces each 5.49 -> 4.84 ms. */
+static int subdivision(int n, int KB, int requested, int p)
+{
+    if (requested <= 0) return 1;
+    int target = choose_partitions(1 << 30, KB, 0); /* what fills the GPU */
+    if (KB <= 4 && target > 2048) target = 2048;
+    const long long most = (n / p) / ((KB >= 64 ? 8LL : 16LL) * KB);
+    const long long sub = target / p < most ? target / p : most;
+    return sub > 1 ? (int)sub : 1;
+}
+
 void spk_plan_destroy(spk_plan *P)
 {
     if (!P) return;
@@ -437,6 +457,7 @@ int spk_plan_build(int n, long long nnz, int ku, int kl, int KB, int is_complex,
     P->mode = mode;
     P->nrhs_max = nrhs_max;
     P->p = p;
+    P->p_user = p;
     P->n_iface = p - 1;
     P->part_start = (int *)malloc(sizeof(int) * (p + 1));
     P->blk_off = (int *)malloc(sizeof(int) * (p + 1));
@@ -548,8 +569,8 @@ static int plan_create(int n, long long nnz, int ku, int kl, int is_complex, int
     const int k = ku > kl ? ku : kl;
     const int KB = spk_choose_block(k < 1 ? 1 : k);
     if (!KB || spk_factor_smem(KB, is_complex, mode) == 0) return SPK_EBAND;
-    const int p = choose_partitions(n, KB, partitions);
-    int *ps = (int *)malloc(sizeof(int) * (p + 1));
+    const int p = choose_partitions(n, KB, partitions), sub = subdivision(n, KB, partitions, p);
+    int *ps = (int *)malloc(sizeof(int) * ((size_t)p * sub + 1));
     if (!ps) return SPK_EMEM;
     /* A partition count the caller asked for gets the reference's layout
      * (spike_solve_analysis: n/p rows each, the remainder in the last one);
@@ -557,9 +578,14 @@ static int plan_create(int n, long long nnz, int ku, int kl, int is_complex, int
      * partitions, since a long last partition's chain would set the time
      * (with many small partitions the remainder can be a hundred blocks). */
     const int nreg = n / p, rem = partitions > 0 ? 0 : n % p;
-    for (int i = 0; i < p; i++) ps[i] = i * nreg + (i < rem ? i : rem);
-    ps[p] = n;
-    const int rc = spk_plan_build(n, nnz, ku, kl, KB, is_complex, mode, p, ps, nrhs_max, stream, stream_alloc, out);
+    for (int i = 0; i < p; i++) {
+        const int s = i * nreg + (i < rem ? i : rem), e = i + 1 < p ? (i + 1) * nreg + (i + 1 < rem ? i + 1 : rem) : n;
+        const int m = (e - s) / sub, more = (e - s) % sub;
+        for (int j = 0; j < sub; j++) ps[(size_t)i * sub + j] = s + j * m + (j < more ? j : more);
+    }
+    ps[(size_t)p * sub] = n;
+    const int rc = spk_plan_build(n, nnz, ku, kl, KB, is_complex, mode, p * sub, ps, nrhs_max, stream, stream_alloc, out);
+    if (rc == SPK_OK) (*out)->p_user = p;
     free(ps);
     return rc;
 }
@@ -569,15 +595,19 @@ size_t spk_solve_footprint(int n, long long nnz, int k, int nrhs, int is_complex
 {
     const int KB = spk_choose_block(k < 1 ? 1 : k);
     if (!KB || n <= 0) return 0;
-    const int p = choose_partitions(n, KB, partitions);
-    const int nreg = n / p;
+    int p = choose_partitions(n, KB, partitions);
+    const int nreg = n / p, sub = subdivision(n, KB, partitions, p);
+    /* blocks of m rows in `pieces` balanced pieces: m % pieces of them hold one row more */
+#define PIECES(m, pieces)                                                                                       \
+    (((m) % (pieces)) * (((m) / (pieces) + 1 + KB - 1) / KB) +                                                  \
+     ((pieces) - (m) % (pieces)) * (((m) / (pieces) + KB - 1) / KB))
     long long blocks;
     if (partitions > 0) /* the reference's layout (plan_create) */
-        blocks = (long long)(p - 1) * ((nreg + KB - 1) / KB) + ((n - (long long)(p - 1) * nreg) + KB - 1) / KB;
-    else { /* balanced: n % p partitions of nreg + 1 rows */
-        const int rem = n % p;
-        blocks = (long long)rem * ((nreg + 1 + KB - 1) / KB) + (long long)(p - rem) * ((nreg + KB - 1) / KB);
-    }
+        blocks = (p - 1) * PIECES((long long)nreg, sub) + PIECES(n - (long long)(p - 1) * nreg, sub);
+    else
+        blocks = PIECES((long long)n, p);
+#undef PIECES
+    p *= sub;
     const long long nif = p > 1 ? p - 1 : 1;
     long long tiles = 0, mtiles = 0;
     for (long long c = nif, l = 0;; l++) {
@@ -613,7 +643,8 @@ static int plan_matches(const spk_plan *P, int n, int ku, int kl, int is_complex
     const int k = ku > kl ? ku : kl;
     const int KB = spk_choose_block(k < 1 ? 1 : k);
     return P->n == n && P->KB == KB && P->is_complex == is_complex && P->mode == mode &&
-           P->p == choose_partitions(n, KB, partitions) && nrhs <= P->nrhs_max;
+           P->p_user == choose_partitions(n, KB, partitions) &&
+           P->p == P->p_user * subdivision(n, KB, partitions, P->p_user) && nrhs <= P->nrhs_max;
 }
 
 /* ------------------------------------------------------------------ */
@@ -754,7 +785,7 @@ static void fill_info(spike_context_t c, const spk_plan *P, const refine_opts *o
 {
     c->info.relres_max = o->relres_max;
     c->info.refine_sweeps = o->sweeps;
-    c->info.partitions = P->p;
+    c->info.partitions = P->p_user;
     c->info.ku = P->ku;
     c->info.kl = P->kl;
     c->info.block = P->KB;
@@ -790,7 +821,8 @@ static int run_device(spike_context_t c, int n, long long nnz, int nrhs, const i
      * call fall back to analysis, a new plan and a second factorization. */
     spk_plan *Q = c->plan;
     if (Q && Q->n == n && Q->nnz == nnz && Q->is_complex == is_complex && Q->mode == c->mode &&
-        Q->p == choose_partitions(n, Q->KB, c->partitions) && chunk0 <= Q->nrhs_max) {
+        Q->p_user == choose_partitions(n, Q->KB, c->partitions) &&
+        Q->p == Q->p_user * subdivision(n, Q->KB, c->partitions, Q->p_user) && chunk0 <= Q->nrhs_max) {
         unsigned e[4];
         Q->twist = Q->twist_cap && c->twist;
         Q->red_fp64 = c->red_fp64 && Q->KB <= 64;
@@ -1013,7 +1045,9 @@ static int host_pipelined(spike_context_t c, int n, long long nnz, int nrhs, con
     spk_plan *Q = c->plan;
     const int chunk = nrhs < RHS_CHUNK ? nrhs : RHS_CHUNK;
     if (!Q || Q->n != n || Q->nnz != nnz || Q->is_complex != cplx || Q->mode != c->mode || !Q->twist_cap || !c->twist ||
-        Q->p != choose_partitions(n, Q->KB, c->partitions) || chunk > Q->nrhs_max || Q->p < PIPE_RANGES ||
+        Q->p_user != choose_partitions(n, Q->KB, c->partitions) ||
+        Q->p != Q->p_user * subdivision(n, Q->KB, c->partitions, Q->p_user) || chunk > Q->nrhs_max ||
+        Q->p < PIPE_RANGES ||
         Q->KB < 16 || Q->KB > 64 ||
         nnz < (8LL << 20) || c->timing)
         return SPK_EARG;

@@ -82,6 +82,7 @@ typedef struct spk_sysref {
 typedef struct spk_plan {
     /* problem */
     int n, nrhs_max, ku, kl, KB, p;
+    int p_user; /* the partition count the caller sees: p, or what p subdivides (plan_create) */
     int is_complex, mode;
     long long nnz;
     /* schedule (host copies) */

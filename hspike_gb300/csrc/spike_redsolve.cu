@@ -14,8 +14,11 @@
 //             updated from one side each -- g^0 by its left odd neighbour, g^1 by
 //             its right one -- so a segment between two surviving blocks
 //             (every 2^s-th) needs nothing from the next segment until only
-//             those survivors are left: s levels cost s barriers of one CTA
-//             instead of s launches.
+//             those survivors are left: s levels cost a few barriers of one
+//             CTA instead of 2 s launches.  Whole solves against one launch per
+//             level and direction: n = 1,000, k = 2 (249 interfaces, one CTA)
+//             655 -> 247 us; n = 300,007, k = 8 (2,431 interfaces, three tiers)
+//             888 -> 586 us.
 //   KB >= 32  k_crq_*: one launch per level and direction, a cluster of CTAs per
 //             block: four rows of the products per warp, every operand of both
 //             products requested before the first is used, the vector between

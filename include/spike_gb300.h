@@ -33,7 +33,8 @@ typedef struct spike_factor_s *spike_factor_t;
 
 /* ---- options (spike_set_option) ---- */
 #define SPIKE_OPT_PRECISION 0      /* SPIKE_PRECISION_MIXED (default) or _FP64 */
-#define SPIKE_OPT_PARTITIONS 1     /* 0 = automatic (default), else p */
+#define SPIKE_OPT_PARTITIONS 1     /* 0 = automatic (default), else p (partitions long enough to leave the GPU
+                                      idle are split further inside; p's boundaries stay partition boundaries) */
 #define SPIKE_OPT_MAX_REFINE 2     /* correction sweeps after the first solve (default 3) */
 #define SPIKE_OPT_TOLERANCE 3      /* relative residual target (default 1e-12) */
 #define SPIKE_OPT_REDUCED_REFINE 4 /* FP64 refinement sweeps on the reduced system (default 2 mixed, 1 FP64) */
