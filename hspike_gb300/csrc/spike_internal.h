@@ -213,6 +213,10 @@ int spk_residual(const spk_plan *P, const int *d_rowptr, const int *d_colind, co
                  const void *d_x, const void *d_b, void *d_r, int nrhs, int want_bnorm, double *d_norms,
                  void *stream);
 
+/* the same for a full band with several columns (spike_residual.cu) */
+int spk_residual_slices(const spk_plan *P, const double *d_aij, const double *d_x, const double *d_b, double *d_r,
+                        int nrhs, int want_bnorm, double *d_norms, void *stream);
+
 /* Batch residual in FP64 / complex128 over the systems of a group, one CTA
  * per chunk of rows of one system (d_chunks: {system, first local row} pairs,
  * rows_per_chunk rows each).  have_x = 0: r = b (x is zero); 1: r = b - A x.

@@ -1,0 +1,165 @@
+// spike_slices.cuh -- FP64 dot products on the tensor cores, exactly.
+//
+// GB300 retires 2 FP64 multiply-adds per clock and SM, its tensor cores about
+// a thousand FP16 ones.  An FP64 value that shares a power-of-two scale with
+// the other values of its row (left operand) or column (right operand) is a
+// 62-bit integer, X = v 2^(61 - E) with |v| < 2^(E+1), and that integer is eight
+// signed byte digits, X = sum_i d_i 256^(7-i), -128 <= d_i <= 127.  Digits are
+// exact in FP16 and their products exact in FP32, so
+//
+//     sum_k X_k Y_k = sum_s 256^(14-s) sum_{i+j=s} sum_k d_i(X_k) d_j(Y_k)
+//
+// takes one m16n8k16 product per digit pair with the FP32 accumulator of each
+// s exact as long as it holds at most SL_FLUSH k steps: 8 pairs x 2^14 x 128
+// <= 2^24 at s = 7.  The pairs with s >= 8 are left out: together they stay
+// below 2^-58 of the two scales' product, while an FP64 sum rounds at 2^-53 of
+// the partial sums (the splitting is Ozaki, Ogita, Oishi, Rump's, Numer.
+// Algorithms 59, 2012, with the digits taken by bytes).
+//
+// What the scales could lose -- values far below the largest of their row or
+// column -- is watched by one more product, of |x| and |y| as powers of two:
+// where sum |x||y| is below SL_GUARD of the scales' product the caller forms
+// that result in FP64 as before.
+#pragma once
+#include <cuda_fp16.h>
+
+#include "spike_common.cuh"
+
+constexpr int SL_D = 8;              // digits
+constexpr int SL_FLUSH = 8;          // k steps (of 16) an FP32 accumulator holds exactly
+constexpr float SL_GUARD = 0.015625f; // 2^-6 (the magnitudes are rounded down to powers of two)
+
+// biased exponent of |v| (0 for zero and subnormals, 0x7ff for inf and NaN)
+__device__ __forceinline__ int sl_exp(double v) { return (int)(((unsigned)__double2hiint(v) >> 20) & 0x7ffu); }
+
+// the 64-bit word whose bytes are the digits of v (+128 each) at scale exponent
+// E (biased; every value of the row has exponent <= E, 64 <= E < 0x7ff; a zero
+// or subnormal v shifts out whole), and |v| 2^-E rounded down to a power of two, in FP16
+__device__ __forceinline__ void sl_split(double v, int E, unsigned &hi, unsigned &lo, unsigned &mag)
+{
+    const unsigned vh = (unsigned)__double2hiint(v), vl = (unsigned)__double2loint(v);
+    const unsigned sh = (unsigned)(E - (int)((vh >> 20) & 0x7ffu));
+    // 53 bits at the top of 62: v 2^(61 - E) where v has exponent E
+    const unsigned mh = __funnelshift_l(vl, (vh & 0xfffffu) | 0x100000u, 9), ml = vl << 9;
+    unsigned long long m = ((unsigned long long)mh << 32) | ml, q;
+    asm("shr.u64 %0, %1, %2;" : "=l"(q) : "l"(m), "r"(sh)); // shifts of 64 and more give 0
+    const long long sg = (long long)((int)vh >> 31);
+    m = (unsigned long long)(((long long)q ^ sg) - sg) + 0x8080808080808080ull;
+    hi = (unsigned)(m >> 32);
+    lo = (unsigned)m;
+    mag = (unsigned)max(15 - (int)sh, 0) << 10;
+}
+
+// digit I (0 = leading) of two values packed as FP16: low half from (hi0, lo0)
+template <int I>
+__device__ __forceinline__ unsigned sl_digit(unsigned hi0, unsigned lo0, unsigned hi1, unsigned lo1)
+{
+    constexpr int B = 3 - (I & 3); // byte within the word
+    const unsigned a = I < 4 ? hi0 : lo0, b = I < 4 ? hi1 : lo1;
+    // bytes a.B and b.B under the exponent of 1024: 1024 + u, exact; then u - 128
+    const unsigned p = (__byte_perm(a, b, B | (B << 4) | ((4 + B) << 8) | ((4 + B) << 12)) & 0x00ff00ffu) | 0x64006400u;
+    const __half2 d = __hsub2(*reinterpret_cast<const __half2 *>(&p), __float2half2_rn(1152.f));
+    return *reinterpret_cast<const unsigned *>(&d);
+}
+
+__device__ __forceinline__ void sl_mma(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1)
+{
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                 "{%0,%1,%2,%3};\n"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// A digits of one k step: a[i] = the m16n8k16 left fragment of digit i, mg = of the magnitudes
+struct SlFragA {
+    unsigned a[SL_D][4], mg[4];
+    // v[r][q]: rows (lane / 4) and (lane / 4) + 8 (r), columns 2 (lane % 4) + {0, 1, 8, 9} (q)
+    __device__ __forceinline__ void split(const double (&v)[2][4], int E0, int E1)
+    {
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                unsigned h0, l0, m0, h1, l1, m1;
+                sl_split(v[r][2 * q], r ? E1 : E0, h0, l0, m0);
+                sl_split(v[r][2 * q + 1], r ? E1 : E0, h1, l1, m1);
+                const int f = r + 2 * q; // fragment registers: (g, lo), (g + 8, lo), (g, hi), (g + 8, hi)
+                a[0][f] = sl_digit<0>(h0, l0, h1, l1);
+                a[1][f] = sl_digit<1>(h0, l0, h1, l1);
+                a[2][f] = sl_digit<2>(h0, l0, h1, l1);
+                a[3][f] = sl_digit<3>(h0, l0, h1, l1);
+                a[4][f] = sl_digit<4>(h0, l0, h1, l1);
+                a[5][f] = sl_digit<5>(h0, l0, h1, l1);
+                a[6][f] = sl_digit<6>(h0, l0, h1, l1);
+                a[7][f] = sl_digit<7>(h0, l0, h1, l1);
+                mg[f] = m0 | (m1 << 16);
+            }
+    }
+};
+
+// one warp's 16 x 8 sums of digit products.  Element e of a lane: row
+// (lane / 4) + 8 (e / 2), column 2 (lane % 4) + e % 2.
+struct SlAcc {
+    float c[SL_D][4], g[4];
+    __device__ __forceinline__ void zero()
+    {
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+#pragma unroll
+            for (int s = 0; s < SL_D; s++) c[s][e] = 0.f;
+            g[e] = 0.f;
+        }
+    }
+    // += the step's products; bfrag(i, r): register r of digit i's right
+    // fragment (i = SL_D: the magnitudes')
+    template <class B> __device__ __forceinline__ void step(const SlFragA &A, B bfrag)
+    {
+        sl_mma(g, A.mg, bfrag(SL_D, 0), bfrag(SL_D, 1));
+#pragma unroll
+        for (int j = 0; j < SL_D; j++) {
+            const unsigned b0 = bfrag(j, 0), b1 = bfrag(j, 1);
+#pragma unroll
+            for (int i = 0; i + j < SL_D; i++) sl_mma(c[i + j], A.a[i], b0, b1);
+        }
+    }
+    // element e as integers, hi 2^32 + lo in units of 256^7
+    __device__ __forceinline__ void total(int e, long long &hi, long long &lo) const
+    {
+        hi = __float2int_rn(c[3][e]);
+        lo = __float2int_rn(c[7][e]);
+#pragma unroll
+        for (int s = 0; s < 3; s++) { // one wide multiply-add each
+            hi += (long long)__float2int_rn(c[s][e]) * (1 << (24 - 8 * s));
+            lo += (long long)__float2int_rn(c[4 + s][e]) * (1 << (24 - 8 * s));
+        }
+    }
+};
+
+// (hi 2^32 + lo) 2^p to FP64, rounded to nearest, with integer instructions
+// (the FP64 pipe is the scarce one); |hi| < 2^60, |lo| < 2^60, and p such that
+// a nonzero result is normal
+__device__ __forceinline__ double sl_round(long long hi, long long lo, int p)
+{
+    hi += lo >> 32;
+    unsigned w0 = (unsigned)lo; // value = hi 2^32 + w0
+    const unsigned neg = hi < 0 ? 0xffffffffu : 0u;
+    if (neg) {
+        w0 = 0u - w0;
+        hi = ~hi + (w0 == 0u ? 1 : 0);
+    }
+    unsigned long long h = (unsigned long long)hi;
+    if (h == 0) {
+        if (w0 == 0u) return 0.0;
+        h = (unsigned long long)w0 << 31;
+        w0 = 0u;
+        p -= 63;
+    }
+    const int z = __clzll((long long)h);
+    unsigned long long m = (h << z) | (z ? ((unsigned long long)w0 << 32) >> (64 - z) : 0ull); // top bit at 63
+    p += 32 - z;
+    const unsigned long long rest = m & 0x7ffull;
+    unsigned long long f = (m >> 11) + (rest > 0x400ull || (rest == 0x400ull && ((m >> 11) & 1)) ? 1 : 0); // 53 bits
+    // f 2^(p + 11): a carry to 2^53 bumps the exponent through the addition
+    const unsigned long long bits = ((unsigned long long)(p + 11 + 52 + 1022) << 52) + f;
+    return __longlong_as_double((long long)(bits | ((unsigned long long)(neg & 0x80000000u) << 32)));
+}
