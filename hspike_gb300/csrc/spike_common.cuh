@@ -1608,6 +1608,82 @@ __device__ __forceinline__ char *smem_align(char *p)
     return (char *)(((uintptr_t)p + 15) & ~(uintptr_t)15);
 }
 
+// ------------------------------------------------------------ dependent launches, levels
+// A kernel of a chain may start while its predecessor is still running
+// (programmatic dependent launch): it does what does not depend on the
+// predecessor and then waits for it (dep_wait).  The first kernel of a chain is
+// launched plainly, and every kernel of the chain waits, so what was complete
+// before the chain is complete for all of it.
+__device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class Kern, class... Args>
+static int launch_dep(Kern k, dim3 grid, int nt, size_t smem, int cluster, bool dep, cudaStream_t st, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(nt);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    int na = 0;
+    if (dep) {
+        at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[na++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[na].id = cudaLaunchAttributeClusterDimension;
+        at[na].val.clusterDim.x = cluster;
+        at[na].val.clusterDim.y = 1;
+        at[na++].val.clusterDim.z = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = na;
+    return cudaLaunchKernelEx(&cfg, k, args...) == cudaSuccess ? SPK_OK : SPK_ECUDA;
+}
+
+constexpr int RS_MAXL = 32;
+
+// the cyclic-reduction levels: blocks, tile offsets of the level arrays (X, Y)
+// and of the odd blocks' M arrays
+struct RsLevels {
+    int L;
+    int cnt[RS_MAXL + 1], off[RS_MAXL + 1], moff[RS_MAXL + 1];
+};
+static inline bool rs_levels(const spk_plan *P, RsLevels &lv)
+{
+    if (P->cr_levels > RS_MAXL) return false;
+    lv.L = P->cr_levels;
+    for (int l = 0; l <= lv.L; l++) {
+        lv.cnt[l] = P->cr_count[l];
+        lv.off[l] = (int)P->cr_off[l];
+        lv.moff[l] = (int)P->cr_moff[l];
+    }
+    return true;
+}
+// Schedule of the levels: the last ones, [top, L], in one CTA, from the first
+// level whose blocks fit its shared memory (all of it when the whole system
+// does, else a quarter: one SM fills its shared memory at roughly 100 GB/s);
+// below them tiers of segments, each as deep as half an SM's shared memory holds.
+// bytes(n, levels, top): shared bytes of a segment of n blocks through `levels` levels.
+template <class B> static inline int rs_schedule(const RsLevels &lv, size_t smem, B bytes, int *tier, int &nt)
+{
+    const int L = lv.L;
+    int lt = 0;
+    if (bytes(lv.cnt[0], L, true) > smem)
+        while (lt < L && bytes(lv.cnt[lt], L - lt, true) > smem / 4) lt++;
+    nt = 0;
+    for (int l = 0; l < lt;) {
+        int s = lt - l;
+        while (s > 1 && bytes((1 << s) + 1, s, false) > smem / 2) s--;
+        tier[nt++] = l;
+        l += s;
+    }
+    tier[nt] = lt;
+    return lt;
+}
+
+
 #define SPK_CHECK_LAUNCH()                                                                      \
     do {                                                                                        \
         cudaError_t e_ = cudaGetLastError();                                                    \

@@ -1074,45 +1074,81 @@ __global__ void __launch_bounds__(QuadBwd<T, KB>::NT)
     cp_async_wait_all();
 }
 
-// Tips of V and W into the interface blocks of the reduced system (FP64):
-//   P_i = V_i bottom, Q_i = W_{i+1} top, X_i = W_i bottom, Y_i = V_{i+1} top.
-template <class T, int KB>
+// Tips of V and W into the interface blocks of the reduced system:
+//   P_i = V_i bottom, Q_i = W_{i+1} top, X_i = W_i bottom, Y_i = V_{i+1} top,
+// as the cyclic reduction's level-0 blocks in its own scalar type S (C*) and,
+// where someone reads them, in FP64 (R*, else NULL): the FP64 residual of small
+// tiles and the records of a sharded solve.
+template <class T, class S, int KB>
 __global__ void k_tips(const int *__restrict__ part_start, const int *__restrict__ blk_off, int p,
-                       const T *__restrict__ gV, const T *__restrict__ gW, typename HighOf<T>::type *RP,
-                       typename HighOf<T>::type *RQ, typename HighOf<T>::type *RX,
+                       const T *__restrict__ gV, const T *__restrict__ gW, S *CP, S *CQ, S *CX, S *CY,
+                       typename HighOf<T>::type *RP, typename HighOf<T>::type *RQ, typename HighOf<T>::type *RX,
                        typename HighOf<T>::type *RY)
 {
     using H = typename HighOf<T>::type;
     constexpr size_t TS = (size_t)KB * KB;
     const int i = blockIdx.x; // interface i between partitions i and i+1
     const int mi = part_start[i + 1] - part_start[i];
-    for (int q = threadIdx.x; q < KB * KB; q += blockDim.x) {
-        const int r = q / KB, c = q - r * KB;
-        // bottom rows of partition i: local row mi - KB + r
-        // (a partition shorter than one tile -- only a batch's one-partition
-        // system, whose spikes are zero -- has no distinct bottom tip)
-        const int lb = mi - KB + r, Jb = lb / KB, rb = lb - Jb * KB;
-        const bool hb = lb >= 0;
-        const size_t ib = hb ? ((size_t)blk_off[i] + Jb) * TS + (size_t)c * KB + rb : 0;
-        // top rows of partition i+1: local row r (block 0)
-        const size_t it = (size_t)blk_off[i + 1] * TS + (size_t)c * KB + r;
-        RP[(size_t)i * TS + q] = hb ? cvt_fast<H, T>(gV[ib]) : sc_zero<H>();
-        RQ[(size_t)i * TS + q] = cvt_fast<H, T>(gW[it]);
-        RX[(size_t)i * TS + q] = (i > 0 && hb) ? cvt_fast<H, T>(gW[ib]) : sc_zero<H>();
-        RY[(size_t)i * TS + q] = (i + 1 < p - 1) ? cvt_fast<H, T>(gV[it]) : sc_zero<H>();
+    // bottom rows of partition i: local row mi - KB + r
+    // (a partition shorter than one tile -- only a batch's one-partition
+    // system, whose spikes are zero -- has no distinct bottom tip);
+    // top rows of partition i+1: local row r (block 0)
+    auto at = [&](int which, int r, int c) {
+        const bool bottom = which == 0 || which == 2, V = which == 0 || which == 3;
+        const int lb = mi - KB + r;
+        if (bottom ? lb < 0 || (which == 2 && i == 0) : which == 3 && i + 1 >= p - 1) return sc_zero<T>();
+        const size_t o = bottom ? ((size_t)blk_off[i] + lb / KB) * TS + (size_t)c * KB + lb % KB
+                                : (size_t)blk_off[i + 1] * TS + (size_t)c * KB + r;
+        return (V ? gV : gW)[o];
+    };
+    auto put = [&](int which, size_t q, T v) {
+        S *C = which == 0 ? CP : which == 1 ? CQ : which == 2 ? CX : CY;
+        if constexpr (std::is_same<S, T>::value)
+            C[q] = v;
+        else
+            C[q] = cvt_fast<S, T>(v);
+        H *R = which == 0 ? RP : which == 1 ? RQ : which == 2 ? RX : RY;
+        if (R) R[q] = cvt_fast<H, T>(v);
+    };
+    if constexpr (KB >= 32) {
+        // the spikes' tiles are column-major: 32 x 32 pieces turn in shared
+        // memory, so both sides are coalesced (blockIdx.y: which block, .z: 32 rows)
+        __shared__ T s[32][33];
+        const int which = blockIdx.y, r0 = blockIdx.z * 32, x = threadIdx.x & 31, y0 = threadIdx.x >> 5;
+        for (int c0 = 0; c0 < KB; c0 += 32) {
+            for (int y = y0; y < 32; y += (int)blockDim.x / 32) s[y][x] = at(which, r0 + x, c0 + y);
+            __syncthreads();
+            for (int y = y0; y < 32; y += (int)blockDim.x / 32)
+                put(which, (size_t)i * TS + (size_t)(r0 + y) * KB + c0 + x, s[x][y]);
+            __syncthreads();
+        }
+    } else {
+        for (int q = threadIdx.x; q < 4 * KB * KB; q += blockDim.x) {
+            const int which = q / (KB * KB), e = q - which * KB * KB;
+            put(which, (size_t)i * TS + e, at(which, e / KB, e % KB));
+        }
     }
 }
 
-template <class T, int KB> int run_tips(spk_plan *P, cudaStream_t st)
+template <class T, class S, int KB> int launch_tips(spk_plan *P, cudaStream_t st)
 {
     using H = typename HighOf<T>::type;
-    if (P->n_iface <= 0) return SPK_OK;
-    k_tips<T, KB><<<P->n_iface, 256, 0, st>>>(P->d_part_start, P->d_blk_off, P->p, (const T *)P->d_V,
-                                              (const T *)P->d_W, (H *)P->d_RP, (H *)P->d_RQ, (H *)P->d_RX,
-                                              (H *)P->d_RY);
+    const bool r = KB <= 16 || P->want_r;
+    k_tips<T, S, KB><<<dim3(P->n_iface, KB >= 32 ? 4 : 1, KB >= 32 ? KB / 32 : 1), KB <= 4 ? 64 : 256, 0, st>>>(
+        P->d_part_start, P->d_blk_off, P->p, (const T *)P->d_V, (const T *)P->d_W, (S *)P->d_crP, (S *)P->d_crQ,
+        (S *)P->d_crX, (S *)P->d_crY, r ? (H *)P->d_RP : nullptr, r ? (H *)P->d_RQ : nullptr,
+        r ? (H *)P->d_RX : nullptr, r ? (H *)P->d_RY : nullptr);
     SPK_CHECK_LAUNCH();
     P->launches++;
+    P->red_direct = 1;
     return SPK_OK;
+}
+template <class T, int KB> int run_tips(spk_plan *P, cudaStream_t st)
+{
+    if (P->n_iface <= 0) return SPK_OK;
+    // the reduced system's scalar type: spk_reduced_factor's choice
+    if (P->mode == SPK_MIXED && P->red_fp64) return launch_tips<T, typename HighOf<T>::type, KB>(P, st);
+    return launch_tips<T, T, KB>(P, st);
 }
 
 // Partitions [part0, part1) of a two-sided plan: their band tiles (the rows'
@@ -1228,12 +1264,10 @@ template <class T, int KB> int run_factor(spk_plan *P, const int *rowptr, const 
                                                           (const T *)P->d_Bhat, (T *)P->d_V, (T *)P->d_W);
         }
         SPK_CHECK_LAUNCH();
-        k_tips<T, KB><<<P->n_iface, 256, 0, st>>>(P->d_part_start, P->d_blk_off, P->p, (const T *)P->d_V,
-                                                  (const T *)P->d_W, (H *)P->d_RP, (H *)P->d_RQ, (H *)P->d_RX,
-                                                  (H *)P->d_RY);
-        SPK_CHECK_LAUNCH();
+        const int rc = run_tips<T, KB>(P, st);
         spk_phase_end(P, st);
-        P->launches += 2;
+        P->launches++;
+        return rc;
     }
     return SPK_OK;
 }

@@ -119,6 +119,8 @@ typedef struct spk_plan {
     void *d_T;                         /* [total_blocks][3][KB][KB]: D, F^T, E per block (row-major) */
     /* reduced system: level-0 quadrant blocks in FP64 (or complex128) */
     void *d_RP, *d_RQ, *d_RX, *d_RY; /* [n_iface][KB][KB] */
+    int want_r;     /* d_RP .. d_RY are read from outside (a sharded solve's records): keep them at every tile size */
+    int red_direct; /* the tips wrote the cyclic reduction's level-0 blocks themselves (else they come from d_RP ..) */
     /* cyclic reduction factors in factor precision */
     int cr_levels;
     int *cr_count;    /* blocks at each level (host), cr_levels+1 entries */

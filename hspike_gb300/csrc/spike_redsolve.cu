@@ -32,48 +32,7 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-// Every kernel of a solve but the first starts while its predecessor is still
-// running (programmatic dependent launch): it fetches the tiles it needs --
-// factors, written long before the solve -- and only then waits for the
-// predecessor's vectors.
-__device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-template <class Kern, class... Args>
-int launch_dep(Kern k, dim3 grid, int nt, size_t smem, int cluster, bool dep, cudaStream_t st, Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(nt);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[2];
-    int na = 0;
-    if (dep) {
-        at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[na++].val.programmaticStreamSerializationAllowed = 1;
-    }
-    if (cluster > 1) {
-        at[na].id = cudaLaunchAttributeClusterDimension;
-        at[na].val.clusterDim.x = cluster;
-        at[na].val.clusterDim.y = 1;
-        at[na++].val.clusterDim.z = 1;
-    }
-    cfg.attrs = at;
-    cfg.numAttrs = na;
-    return cudaLaunchKernelEx(&cfg, k, args...) == cudaSuccess ? SPK_OK : SPK_ECUDA;
-}
-
 // ------------------------------------------------------------ KB <= 16: segments
-constexpr int RS_MAXL = 32;
-
-// the cyclic-reduction levels: blocks, tile offsets of the level arrays (X, Y)
-// and of the odd blocks' M arrays
-struct RsLevels {
-    int L;
-    int cnt[RS_MAXL + 1], off[RS_MAXL + 1], moff[RS_MAXL + 1];
-};
-
 template <class T> struct RsArgs {
     using H = typename HighOf<T>::type;
     const T *X, *Y, *M;
@@ -454,14 +413,8 @@ template <class T, int KB, int NRC> int run_red_solve_s(spk_plan *P, int nrhs, i
         attr = true;
     }
     const int L = P->cr_levels;
-    if (L > RS_MAXL) return SPK_EARG;
     RsLevels lv;
-    lv.L = L;
-    for (int l = 0; l <= L; l++) {
-        lv.cnt[l] = P->cr_count[l];
-        lv.off[l] = (int)P->cr_off[l];
-        lv.moff[l] = (int)P->cr_moff[l];
-    }
+    if (!rs_levels(P, lv)) return SPK_EARG;
     RsArgs<T> A;
     A.X = (const T *)P->d_crX;
     A.Y = (const T *)P->d_crY;
@@ -481,21 +434,8 @@ template <class T, int KB, int NRC> int run_red_solve_s(spk_plan *P, int nrhs, i
     A.nrhs = nrhs;
     const int hy = (nrhs + NRC - 1) / NRC;
     auto bytes = [&](int n, int levels, bool top) { return rs_bytes<T>(n, levels, KB, NRC, top); };
-    // The last levels, from the first one whose blocks fit one CTA's shared
-    // memory -- or, where the rest would need segments anyway, a quarter of
-    // it: a CTA fills its shared memory at roughly 100 GB/s.
-    int lt = 0;
-    if (bytes(lv.cnt[0], L, true) > SMEM)
-        while (lt < L && bytes(lv.cnt[lt], L - lt, true) > SMEM / 4) lt++;
-    // tiers of segments below them, each as deep as half an SM's shared memory holds
-    int tier[RS_MAXL + 1], nt = 0;
-    for (int l = 0; l < lt;) {
-        int s = lt - l;
-        while (s > 1 && bytes((1 << s) + 1, s, false) > SMEM / 2) s--;
-        tier[nt++] = l;
-        l += s;
-    }
-    tier[nt] = lt;
+    int tier[RS_MAXL + 1], nt;
+    const int lt = rs_schedule(lv, SMEM, bytes, tier, nt);
     bool dep = false; // the first kernel of the solve starts after everything before it
     for (int it = 0; it < (lt == 0 ? 1 : iters); it++) {
         int rc = SPK_OK;
@@ -708,15 +648,34 @@ __global__ void __launch_bounds__(QNT)
     });
 }
 
-// res = g - R u in FP64 with the level-0 quadrant blocks, 32 rows per CTA, a
+// a factor-precision value in FP64, exactly, with integer instructions (subnormals too)
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ cdouble widen(cdouble v) { return v; }
+__device__ __forceinline__ double widen(float v)
+{
+    const unsigned u = __float_as_uint(v);
+    if ((u & 0x7f800000u) == 0x7f800000u) return (double)v;
+    const bool sub = (u & 0x7f800000u) == 0u;
+    const unsigned w = sub ? __float_as_uint(v * 0x1p64f) : u; // a normal number, or zero
+    const unsigned e = (w >> 23) & 0xffu;
+    const unsigned hi = (u & 0x80000000u) |
+                        (e == 0u ? 0u : (((e + (1023u - 127u) - (sub ? 64u : 0u)) << 20) | ((w & 0x7fffffu) >> 3)));
+    return __hiloint2double((int)hi, (int)(w << 29));
+}
+__device__ __forceinline__ cdouble widen(cfloat v) { return {widen(v.re), widen(v.im)}; }
+
+// res = g - R u in FP64 with the level-0 quadrant blocks (spikes' tips: values
+// of the factor precision), 32 rows per CTA, a
 // warp per four rows with its lanes along k: every tile is read once,
 // coalesced (one thread per row walking its KB columns took 281 us at 155
 // interfaces of 64 rows, 16 columns)
-template <class H, int KB, int NRC>
+template <class T, int KB, int NRC>
 __global__ void __launch_bounds__(QNT)
-    k_red_resid(const H *__restrict__ RP, const H *__restrict__ RQ, const H *__restrict__ RX, const H *__restrict__ RY,
-                const H *__restrict__ g, const H *__restrict__ u, H *res, int nif, int nrhs)
+    k_red_resid(const T *__restrict__ RP, const T *__restrict__ RQ, const T *__restrict__ RX, const T *__restrict__ RY,
+                const typename HighOf<T>::type *__restrict__ g, const typename HighOf<T>::type *__restrict__ u,
+                typename HighOf<T>::type *res, int nif, int nrhs)
 {
+    using H = typename HighOf<T>::type;
     using Q = QSolve<H, KB, NRC>;
     constexpr size_t TS = Q::TS;
     __shared__ __align__(16) H sx[NRC * 2 * KB]; // [h]: the two KB-vectors this half's rows meet
@@ -727,16 +686,20 @@ __global__ void __launch_bounds__(QNT)
     const int r0 = rank * QROWS + warp * QRPW, half = rank * QROWS / KB, q0 = r0 - half * KB;
     const bool far = half ? i + 1 < nif : i > 0; // the neighbouring interface exists
     H m[QRPW][2][Q::VW];
-    const H *A0 = (half ? RQ : RP) + (size_t)i * TS, *A1 = (half ? RY : RX) + (size_t)i * TS;
+    const T *A0 = (half ? RQ : RP) + (size_t)i * TS, *A1 = (half ? RY : RX) + (size_t)i * TS;
+    T mt[QRPW][2][Q::VW];
 #pragma unroll
     for (int gq = 0; gq < QRPW; gq++) {
-        vld<H, Q::VW>(m[gq][0], A0 + (size_t)(q0 + gq) * KB + lane * Q::VW);
-        if (far)
-            vld<H, Q::VW>(m[gq][1], A1 + (size_t)(q0 + gq) * KB + lane * Q::VW);
-        else
-#pragma unroll
-            for (int w = 0; w < Q::VW; w++) m[gq][1][w] = sc_zero<H>();
+        vld<T, Q::VW>(mt[gq][0], A0 + (size_t)(q0 + gq) * KB + lane * Q::VW);
+        vld<T, Q::VW>(mt[gq][1], A1 + (size_t)(q0 + gq) * KB + lane * Q::VW);
     }
+#pragma unroll
+    for (int gq = 0; gq < QRPW; gq++)
+#pragma unroll
+        for (int w = 0; w < Q::VW; w++) {
+            m[gq][0][w] = widen(mt[gq][0][w]);
+            m[gq][1][w] = far ? widen(mt[gq][1][w]) : sc_zero<H>();
+        }
     dep_launch();
     dep_wait();
     for (int q = threadIdx.x; q < NRC * 2 * KB; q += QNT) {
@@ -788,9 +751,8 @@ template <class T, int KB, int NRC> int run_red_solve_q(spk_plan *P, int nrhs, i
         P->launches += 2 * L + 1;
         if (it + 1 < iters) {
             constexpr int RC = NRC > 4 ? 4 : NRC;
-            if (launch_dep(k_red_resid<H, KB, RC>, dim3(P->n_iface * Q::CS, (nrhs + RC - 1) / RC), QNT, 0, 1, true, st,
-                           (const H *)P->d_RP, (const H *)P->d_RQ, (const H *)P->d_RX, (const H *)P->d_RY,
-                           (const H *)P->d_g, (const H *)P->d_u, (H *)P->d_rr, P->n_iface, nrhs) != SPK_OK)
+            if (launch_dep(k_red_resid<T, KB, RC>, dim3(P->n_iface * Q::CS, (nrhs + RC - 1) / RC), QNT, 0, 1, true, st,
+                           (const T *)P->d_crP, (const T *)P->d_crQ, cX, cY, (const H *)P->d_g, (const H *)P->d_u, (H *)P->d_rr, P->n_iface, nrhs) != SPK_OK)
                 return SPK_ECUDA;
             P->launches++;
         }

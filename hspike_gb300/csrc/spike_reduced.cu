@@ -335,11 +335,221 @@ __global__ void __launch_bounds__(NTOf<KB>::value)
     tc_each<KB>(acc, [&](int r, int c, float v) { out[r * KB + c] = (base ? base[r * KB + c] : 0.f) - v; });
 }
 
+// ------------------------------------------------------------ KB <= 16: segments of several levels
+// The factorization's counterpart of the solve's segments (spike_redsolve.cu):
+// of an even block's four results P' and X' depend on its left odd neighbour
+// only, Q' and Y' on its right one, so a CTA takes a segment between two
+// survivors through several levels on its own -- a group of GL lanes per tile
+// product, everything in shared memory.  One launch per level and parity took
+// 127 us for 2,431 interfaces of 8-row tiles (11 levels of two launches of
+// 3.5 to 6 us each and four conversions); 42 us.
+template <class T, int KB> struct RfCfg {
+    static constexpr int TS = KB * KB;
+    static constexpr int GL = TS < 32 ? TS : 32; // lanes per tile
+    static constexpr int EPL = TS / GL;          // elements per lane
+    static constexpr int SCR = TS + 4 * KB;      // scratch elements per group: a tile, the pivot rows and columns
+};
+
+template <class T, int KB, int NT>
+__global__ void __launch_bounds__(NT)
+    k_rf_seg(T *gP, T *gQ, T *gX, T *gY, T *gM, const __grid_constant__ RsLevels lv, int l0, int l1, int top,
+             unsigned *err)
+{
+    using C = RfCfg<T, KB>;
+    constexpr int TS = C::TS, GL = C::GL, EPL = C::EPL, NG = NT / GL;
+    const int s = l1 - l0, full = 1 << s;
+    int b = top ? 0 : (int)blockIdx.x << s;
+    const int left = lv.cnt[l0] - b, n0 = top || left <= full ? left : full + 1;
+    int end = top || left <= full ? 1 << 30 : full; // the right survivor: only its P' and X' are ours
+    const bool first = b == 0;
+    extern __shared__ __align__(16) char smraw[];
+    T *cur = (T *)smraw;                        // P, Q, X, Y of the level's blocks
+    T *nxt = cur + (size_t)4 * n0 * TS;         // of the next level's
+    T *sM = nxt + (size_t)4 * ((n0 + 1) / 2) * TS; // four tiles per odd block
+    T *scr = sM + (size_t)4 * (n0 / 2 > 0 ? n0 / 2 : 1) * TS;
+    const int grp = threadIdx.x / GL, e0 = threadIdx.x % GL;
+    const unsigned gm = GL == 32 ? 0xffffffffu : ((1u << GL) - 1u) << ((threadIdx.x & 31) / GL * GL);
+    T *tmp = scr + (size_t)grp * C::SCR, *piv = tmp + TS;
+    bool ok = true;
+
+    auto er = [&](int q) { return (e0 + q * GL) / KB; };
+    auto ec = [&](int q) { return (e0 + q * GL) % KB; };
+    // acc -= A B (dense shared tiles)
+    auto msub_t = [&](T (&acc)[EPL], const T *A, const T *B) {
+#pragma unroll
+        for (int q = 0; q < EPL; q++)
+#pragma unroll
+            for (int k = 0; k < KB; k++) acc[q] = msub(acc[q], A[er(q) * KB + k], B[k * KB + ec(q)]);
+    };
+    auto madd_t = [&](T (&acc)[EPL], const T *A, const T *B) {
+#pragma unroll
+        for (int q = 0; q < EPL; q++)
+#pragma unroll
+            for (int k = 0; k < KB; k++) acc[q] = madd(acc[q], A[er(q) * KB + k], B[k * KB + ec(q)]);
+    };
+    auto put = [&](T *d, const T (&v)[EPL]) {
+#pragma unroll
+        for (int q = 0; q < EPL; q++) d[e0 + q * GL] = v[q];
+    };
+    // M = D^{-1} of the block with tiles P, Q, by quadrants: S = I - Q P, M11 =
+    // S^{-1}, M10 = -M11 Q, M01 = -P M11, M00 = I - P M10
+    auto odd = [&](const T *P, const T *Q, T *M, T *out) {
+        T a[EPL];
+#pragma unroll
+        for (int q = 0; q < EPL; q++) a[q] = er(q) == ec(q) ? sc_one<T>() : sc_zero<T>();
+        msub_t(a, Q, P);
+        // Gauss-Jordan without pivoting, row and column of the pivot through shared memory
+        for (int j = 0; j < KB; j++) {
+            T *row = piv + (j & 1) * 2 * KB, *col = row + KB;
+#pragma unroll
+            for (int q = 0; q < EPL; q++) {
+                if (er(q) == j) row[ec(q)] = a[q];
+                if (ec(q) == j) col[er(q)] = a[q];
+            }
+            __syncwarp(gm);
+            const T p = col[j];
+            if (!sc_finite_nonzero(p)) ok = false;
+            const T pr = sc_frcp(p);
+#pragma unroll
+            for (int q = 0; q < EPL; q++) {
+                const T bv = row[ec(q)] * pr, av = col[er(q)];
+                a[q] = ec(q) == j ? (er(q) == j ? pr : -(av * pr)) : er(q) == j ? bv : msub(a[q], av, bv);
+            }
+        }
+        put(M + 3 * TS, a);
+        put(out + 3 * TS, a);
+        __syncwarp(gm);
+        T z[EPL];
+#pragma unroll
+        for (int q = 0; q < EPL; q++) a[q] = z[q] = sc_zero<T>();
+        msub_t(a, M + 3 * TS, Q);
+        msub_t(z, P, M + 3 * TS);
+        put(M + 2 * TS, a);
+        put(out + 2 * TS, a);
+        put(M + TS, z);
+        put(out + TS, z);
+        __syncwarp(gm);
+#pragma unroll
+        for (int q = 0; q < EPL; q++) a[q] = er(q) == ec(q) ? sc_one<T>() : sc_zero<T>();
+        msub_t(a, P, M + 2 * TS);
+        put(M, a);
+        put(out, a);
+    };
+
+    dep_launch();
+    dep_wait();
+    {
+        const size_t o = (size_t)(lv.off[l0] + b) * TS;
+        for (int q = threadIdx.x; q < n0 * TS; q += NT) {
+            cur[q] = gP[o + q];
+            cur[(size_t)n0 * TS + q] = gQ[o + q];
+            cur[(size_t)2 * n0 * TS + q] = gX[o + q];
+            cur[(size_t)3 * n0 * TS + q] = gY[o + q];
+        }
+    }
+    __syncthreads();
+    int nl = n0;
+    for (int l = l0; l < l1; l++) {
+        const int nodd = nl >> 1, nn = (nl + 1) >> 1;
+        const T *P = cur, *Q = P + (size_t)nl * TS, *X = Q + (size_t)nl * TS, *Y = X + (size_t)nl * TS;
+        for (int j = grp; j < nodd; j += NG)
+            odd(P + (size_t)(2 * j + 1) * TS, Q + (size_t)(2 * j + 1) * TS, sM + (size_t)j * 4 * TS,
+                gM + (size_t)(lv.moff[l] + b / 2 + j) * 4 * TS);
+        __syncthreads();
+        // P' = P_i - X_i (M01 Y)_{i-1}, Q' = Q_i - Y_i (M10 X)_{i+1}, X' = -X_i (M00 X)_{i-1}, Y' = -Y_i (M11 Y)_{i+1}
+        for (int it = grp; it < 4 * nn; it += NG) {
+            const int a = it >> 2, w = it & 3, i = 2 * a;
+            const bool lft = w == 0 || w == 2;
+            const int j = lft ? i - 1 : i + 1;
+            T v[EPL];
+#pragma unroll
+            for (int q = 0; q < EPL; q++)
+                v[q] = w == 0 ? P[(size_t)i * TS + e0 + q * GL] : w == 1 ? Q[(size_t)i * TS + e0 + q * GL] : sc_zero<T>();
+            if (lft ? j >= 0 : j < nl) {
+                const T *M = sM + (size_t)(j >> 1) * 4 * TS;
+                T m[EPL];
+#pragma unroll
+                for (int q = 0; q < EPL; q++) m[q] = sc_zero<T>();
+                madd_t(m, M + (w == 0 ? 1 : w == 1 ? 2 : w == 2 ? 0 : 3) * TS,
+                       (w == 0 || w == 3 ? Y : X) + (size_t)j * TS);
+                put(tmp, m);
+                __syncwarp(gm);
+                msub_t(v, (lft ? X : Y) + (size_t)i * TS, tmp);
+                __syncwarp(gm); // tmp is free again
+            }
+            put(nxt + (size_t)(w * nn + a) * TS, v);
+            if (lft ? (i > 0 || first) : i < end)
+                put((w == 0 ? gP : w == 1 ? gQ : w == 2 ? gX : gY) + (size_t)(lv.off[l + 1] + b / 2 + a) * TS, v);
+        }
+        __syncthreads();
+        T *sw = cur;
+        cur = nxt;
+        nxt = sw;
+        nl = nn;
+        b >>= 1;
+        end >>= 1;
+    }
+    if (top && grp == 0) odd(cur, cur + TS, sM, gM + (size_t)lv.moff[lv.L] * 4 * TS); // the last single block
+    if (!ok && e0 == 0) atomicOr(err, SPK_DEV_ERR_PIVOT);
+}
+
+template <class T, int KB> int run_red_factor_s(spk_plan *P, cudaStream_t st)
+{
+    using C = RfCfg<T, KB>;
+    constexpr int NT = 256, NTT = 512;
+    constexpr size_t SMEM = 220 * 1024;
+    static bool attr = false;
+    if (!attr) {
+        if (cudaFuncSetAttribute(k_rf_seg<T, KB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) !=
+                cudaSuccess ||
+            cudaFuncSetAttribute(k_rf_seg<T, KB, NTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) !=
+                cudaSuccess)
+            return SPK_ECUDA;
+        attr = true;
+    }
+    RsLevels lv;
+    if (!rs_levels(P, lv)) return SPK_EARG;
+    auto bytes = [](int n, int, bool top) {
+        const size_t tiles = 4 * (size_t)n + 4 * ((n + 1) / 2) + 4 * (size_t)(n / 2 > 0 ? n / 2 : 1);
+        return (tiles * C::TS + (size_t)(top ? NTT : NT) / C::GL * C::SCR) * sizeof(T) + 16;
+    };
+    int tier[RS_MAXL + 1], nt;
+    const int lt = rs_schedule(lv, SMEM, bytes, tier, nt);
+    bool dep = false;
+    auto run = [&](auto kern, int grid, int nthr, size_t smem, int l0, int l1, int top) {
+        const int rc = launch_dep(kern, dim3(grid), nthr, smem, 1, dep, st, (T *)P->d_crP, (T *)P->d_crQ,
+                                  (T *)P->d_crX, (T *)P->d_crY, (T *)P->d_crM, lv, l0, l1, top, P->d_err);
+        dep = true;
+        P->launches++;
+        return rc;
+    };
+    for (int q = 0; q < nt; q++) {
+        const int l0 = tier[q], l1 = tier[q + 1], s = l1 - l0;
+        if (run(k_rf_seg<T, KB, NT>, (lv.cnt[l0] + (1 << s) - 1) >> s, NT, bytes((1 << s) + 1, s, false), l0, l1, 0) !=
+            SPK_OK)
+            return SPK_ECUDA;
+    }
+    return run(k_rf_seg<T, KB, NTT>, 1, NTT, bytes(lv.cnt[lt], lv.L - lt, true), lt, lv.L, 1);
+}
+
 template <class T, int KB> int run_red_factor(spk_plan *P, cudaStream_t st)
 {
     using S = RedSmem<T, KB>;
     constexpr int NT = NTOf<KB>::value;
     constexpr size_t TS = (size_t)KB * KB;
+    using H = typename HighOf<T>::type;
+    if (!P->red_direct) { // the blocks come in FP64 (a sharded solve's records)
+        const long long c0 = (long long)P->n_iface * TS;
+        k_red_cvt<T><<<256, 256, 0, st>>>((const H *)P->d_RP, (T *)P->d_crP, c0);
+        k_red_cvt<T><<<256, 256, 0, st>>>((const H *)P->d_RQ, (T *)P->d_crQ, c0);
+        k_red_cvt<T><<<256, 256, 0, st>>>((const H *)P->d_RX, (T *)P->d_crX, c0);
+        k_red_cvt<T><<<256, 256, 0, st>>>((const H *)P->d_RY, (T *)P->d_crY, c0);
+        SPK_CHECK_LAUNCH();
+        P->launches += 4;
+    }
+    if constexpr (KB <= 16) {
+        return run_red_factor_s<T, KB>(P, st);
+    } else {
     // FP32 factors with 64- or 128-row tiles: the block products on the tensor cores
     constexpr bool TC = std::is_same<T, float>::value && (KB == 64 || KB == 128);
     static bool attr = false;
@@ -362,14 +572,6 @@ template <class T, int KB> int run_red_factor(spk_plan *P, cudaStream_t st)
         else
             k_cr_odd<T, KB><<<count, NT, S::bytes, st>>>(Pp, Qp, first, stride, Mo, P->d_err);
     };
-    using H = typename HighOf<T>::type;
-    const long long c0 = (long long)P->n_iface * TS;
-    k_red_cvt<T><<<256, 256, 0, st>>>((const H *)P->d_RP, (T *)P->d_crP, c0);
-    k_red_cvt<T><<<256, 256, 0, st>>>((const H *)P->d_RQ, (T *)P->d_crQ, c0);
-    k_red_cvt<T><<<256, 256, 0, st>>>((const H *)P->d_RX, (T *)P->d_crX, c0);
-    k_red_cvt<T><<<256, 256, 0, st>>>((const H *)P->d_RY, (T *)P->d_crY, c0);
-    SPK_CHECK_LAUNCH();
-    P->launches += 4;
     T *cP = (T *)P->d_crP, *cQ = (T *)P->d_crQ, *cX = (T *)P->d_crX, *cY = (T *)P->d_crY, *cM = (T *)P->d_crM;
     for (int l = 0; l < P->cr_levels; l++) {
         const int cnt = P->cr_count[l];
@@ -398,6 +600,7 @@ template <class T, int KB> int run_red_factor(spk_plan *P, cudaStream_t st)
         P->launches++;
     }
     return SPK_OK;
+    }
 }
 
 #define SPK_KB_SWITCH(FN, T, ...)                                                                               \

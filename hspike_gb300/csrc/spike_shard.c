@@ -234,6 +234,7 @@ static int shard_plans(shard_t *S, int KB)
     int rc = spk_plan_build(nl, S->nnz_loc, KB, KB, KB, 0, c->mode, pl, ps, nr, c->stream, 0, &S->P);
     free(ps);
     TRY(rc);
+    S->P->want_r = 1; /* its interface blocks travel as FP64 records */
     const size_t vb = sizeof(double) * (size_t)nl * nr;
     TRY(spk_malloc((void **)&S->d_b, vb));
     TRY(spk_malloc((void **)&S->d_x, vb));
