@@ -418,6 +418,8 @@ template <class T, int KB, int NT> struct Tile {
         else
             return inverse_r1(s, buf);
     }
+    // the same by halves in a whole tile of scratch (ELEMS elements)
+    __device__ __forceinline__ bool inverse_blk(Reg &s, T *tile) const;
 
     // Blocked Gauss-Jordan with 4 x 4 pivot blocks, each the sub-tile of one
     // thread.  With P the pivot block, U the pivot columns, B the pivot rows,
@@ -676,8 +678,6 @@ template <class T, int KB> struct Tile88 {
     static constexpr int ELEMS = KB * LD;
     static constexpr int ACTIVE = 64;
     static constexpr int NT = 64;
-    static constexpr int INV_HALF = 12 * KB + 16;
-    static constexpr int INV_BUF = 2 * INV_HALF + KB;
 
     using Reg = T[TR][TC];
 
@@ -826,152 +826,8 @@ template <class T, int KB> struct Tile88 {
         mm_tA<true, 4, LDA, LDB>(acc, At, B);
     }
 
-    // In-place Gauss-Jordan inverse without pivoting, blocked by 4 x 4 pivot
-    // blocks: the update of Tile::inverse_b4 (S <- S - U'V', U' = pivot
-    // columns - I on the pivot rows, V' = P^{-1} (pivot rows + I on the pivot
-    // columns)) on this layout.  Pivot block q covers rows and columns
-    // 4q .. 4q+3: its rows are register rows 4 (q & 1) .. +3 of sub-tile row
-    // q / 2, its columns register columns 4 (q / 8) .. +3 of sub-tile column
-    // q & 7.  Rows are scaled to a unit diagonal first and the inverse's
-    // columns back after.  buf: INV_BUF elements of shared memory (16-byte
-    // aligned).  All threads must call; false in every thread on a zero or
-    // non-finite pivot.  The register offsets of each step are template
-    // arguments, so the sub-tile never leaves the registers.
-    __device__ __forceinline__ bool inverse(Reg &s, T *buf) const
-    {
-        bool ok = true;
-        T *dg = buf + 2 * INV_HALF; // the diagonal, KB entries
-        // diagonal entry (c, c), c = h*32 + tx*4 + j, sits in sub-tile row
-        // 4h + tx/2, register row 4 (tx & 1) + j, register column 4h + j
-        const bool odd = (tx & 1) != 0;
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-            if (ty == 4 * h + (tx >> 1)) {
-                T d[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) d[j] = reg_sel(odd, s[4 + j][4 * h + j], s[j][4 * h + j]);
-                vst<T, 4>(dg + h * HALF + tx * 4, d);
-            }
-        __syncthreads();
-        {
-            T dr[TR];
-            vld<T, TR>(dr, dg + row(0));
-#pragma unroll
-            for (int i = 0; i < TR; i++) {
-                if (!sc_finite_nonzero(dr[i])) ok = false;
-                const T rr = sc_rcp_fast(dr[i]);
-#pragma unroll
-                for (int jj = 0; jj < TC; jj++) s[i][jj] = s[i][jj] * rr;
-            }
-        }
-        // q = 2 q2 + HQ; pivot columns in register columns 4..7 from q = 8 on
-        for (int q2 = 0; q2 < KB / 16; q2++) {
-            inv_step<false, 0>(s, buf, q2, ok);
-            inv_step<false, 1>(s, buf, q2, ok);
-        }
-        for (int q2 = KB / 16; q2 < KB / 8; q2++) {
-            inv_step<true, 0>(s, buf, q2, ok);
-            inv_step<true, 1>(s, buf, q2, ok);
-        }
-        // columns of the inverse back by the diagonal: S^{-1} = (D^{-1} S)^{-1} D^{-1}
-        {
-            T dc[TC];
-            ld_row(dc, dg);
-#pragma unroll
-            for (int jj = 0; jj < TC; jj++) {
-                const T rc = sc_rcp_fast(dc[jj]);
-#pragma unroll
-                for (int i = 0; i < TR; i++) s[i][jj] = s[i][jj] * rc;
-            }
-        }
-        __syncthreads();
-        return __syncthreads_and(ok ? 1 : 0) != 0;
-    }
-
-    // one 4 x 4 pivot block of inverse(): q = 2 q2 + HQ, its rows register
-    // rows 4 HQ .. 4 HQ + 3 of sub-tile row q2, its columns register columns
-    // (HI ? 4 : 0) .. +3 of sub-tile column q & 7.  The eight owners of the
-    // pivot rows are one quarter-warp: each takes the pivot block P from its
-    // owner by shuffles, inverts it (the same steps in all eight, no barrier)
-    // and forms its own columns of V' = P^{-1} (pivot rows + I); the owners of
-    // the pivot columns publish U'.  One barrier, then every thread applies
-    // S <- S - U' V' to its sub-tile.
-    template <bool HI, int HQ> __device__ __forceinline__ void inv_step(Reg &s, T *buf, int q2, bool &ok) const
-    {
-        constexpr int CO = HI ? 4 : 0, RO = 4 * HQ;
-        const int q = 2 * q2 + HQ;
-        T *cbuf = buf + HQ * INV_HALF; // [KB][4] pivot columns U'
-        T *vbuf = cbuf + 4 * KB;       // [4][KB] V'
-        const bool rown = ty == q2, cown = tx == (q & 7);
-        if (rown) {
-            const int lane = threadIdx.x & 31;
-            const unsigned qmask = 0xffu << (lane & 24);
-            const int src = (lane & 24) + (q & 7); // the pivot block's owner in this quarter-warp
-            T pinv[4][4];
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) pinv[a][b] = __shfl_sync(qmask, s[RO + a][CO + b], src);
-#pragma unroll
-            for (int k = 0; k < 4; k++) { // unblocked Gauss-Jordan in registers
-                const T piv = pinv[k][k];
-                if (!sc_finite_nonzero(piv)) ok = false;
-                const T pr = sc_rcp_fast(piv);
-#pragma unroll
-                for (int b = 0; b < 4; b++)
-                    if (b != k) pinv[k][b] = pinv[k][b] * pr;
-#pragma unroll
-                for (int a = 0; a < 4; a++)
-                    if (a != k) {
-                        const T f = pinv[a][k];
-#pragma unroll
-                        for (int b = 0; b < 4; b++)
-                            if (b != k) pinv[a][b] = msub(pinv[a][b], f, pinv[k][b]);
-                        pinv[a][k] = -(f * pr);
-                    }
-                pinv[k][k] = pr;
-            }
-#pragma unroll
-            for (int tt = 0; tt < 4; tt++) {
-                T vrow[TC];
-#pragma unroll
-                for (int jj = 0; jj < TC; jj++) {
-                    T acc = sc_zero<T>();
-#pragma unroll
-                    for (int a = 0; a < 4; a++) {
-                        const T bb = (cown && jj == CO + a) ? s[RO + a][jj] + sc_one<T>() : s[RO + a][jj];
-                        acc = madd(acc, pinv[tt][a], bb);
-                    }
-                    vrow[jj] = acc;
-                }
-                st_row(vbuf + tt * KB, vrow);
-            }
-        }
-        if (cown) {
-#pragma unroll
-            for (int i = 0; i < TR; i++) {
-                T u[4];
-#pragma unroll
-                for (int t = 0; t < 4; t++) u[t] = (rown && i == RO + t) ? s[i][CO + t] - sc_one<T>() : s[i][CO + t];
-                vst<T, 4>(cbuf + row(i) * 4, u);
-            }
-        }
-        __syncthreads();
-        T u[TR][4], v[4][TC];
-#pragma unroll
-        for (int i = 0; i < TR; i++) vld<T, 4>(u[i], cbuf + row(i) * 4);
-#pragma unroll
-        for (int t = 0; t < 4; t++) ld_row(v[t], vbuf + t * KB);
-#pragma unroll
-        for (int i = 0; i < TR; i++)
-#pragma unroll
-            for (int jj = 0; jj < TC; jj++) {
-                T acc = s[i][jj];
-#pragma unroll
-                for (int t = 0; t < 4; t++) acc = msub(acc, u[i][t], v[t][jj]);
-                s[i][jj] = acc;
-            }
-    }
+    // in-place inverse by halves in a whole tile of scratch (ELEMS elements)
+    __device__ __forceinline__ bool inverse_blk(Reg &s, T *tile) const;
 };
 
 // ------------------------------------------------------------ one warp per tile
@@ -1130,6 +986,139 @@ template <class T, int KB> struct TileW {
         return __all_sync(FULL, ok) != 0;
     }
 };
+
+// ------------------------------------------------------------ blocked inverse in shared memory
+// In-place inverse without pivoting of an N x N FP32 tile (N = 32, 64, row stride LD) in shared memory, by halves: with H11 = A11^{-1}, U = A21 H11,
+// T = H11 A12 and H22 = (A22 - U A12)^{-1},
+//     G12 = -T H22,  G21 = -H22 U,  G11 = H11 - G12 U.
+// The 32-row leaves are one warp's Gauss-Jordan on shuffles (TileW, rows scaled
+// to a unit diagonal); everything else is products that all NT threads share,
+// where a blocked Gauss-Jordan over the whole tile pays a barrier per four
+// pivots.  One 64-row tile on an idle SM: 16,600 clocks on 64 threads, 13,400 on
+// 256, against 20,900 and 15,700; the elimination chains of n = 2,000,000, k = 64
+// (3.4 of them per SM) 2.26 -> 1.92 ms.  At 128 rows and 1,024 threads (64
+// registers each) the leaves spill and Gauss-Jordan stays faster.  All NT
+// threads call, the tile complete in shared memory before and after.
+// products of h x h blocks (row stride LD) on TT threads, TR x TC elements each
+template <int h, int TT, int LD> struct BlkMul {
+    static constexpr int PER = h * h / TT;
+    static constexpr int TC = PER >= 8 ? 4 : PER >= 4 ? 2 : 1;
+    static constexpr int TR = PER / TC;
+    static constexpr int TX = h / TC;
+    static_assert(PER >= 1 && PER * TT == h * h, "whole sub-tiles");
+    using Acc = float[TR][TC];
+    // acc = A B; t: this thread's index among the TT
+    static __device__ __forceinline__ void mul(int t, Acc &acc, const float *A, const float *B)
+    {
+        const int r0 = t / TX * TR, c0 = t % TX * TC;
+#pragma unroll
+        for (int i = 0; i < TR; i++)
+#pragma unroll
+            for (int j = 0; j < TC; j++) acc[i][j] = 0.f;
+#pragma unroll 2
+        for (int k = 0; k < h; k += 4) {
+            float a[TR][4];
+#pragma unroll
+            for (int i = 0; i < TR; i++) vld<float, 4>(a[i], A + (r0 + i) * LD + k);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                float b[TC];
+                vld<float, TC>(b, B + (k + q) * LD + c0);
+#pragma unroll
+                for (int i = 0; i < TR; i++)
+#pragma unroll
+                    for (int j = 0; j < TC; j++) acc[i][j] = fmaf(a[i][q], b[j], acc[i][j]);
+            }
+        }
+    }
+    // D = acc or -acc; ADD: D += that
+    template <bool ADD, bool NEG> static __device__ __forceinline__ void put(int t, float *D, const Acc &acc)
+    {
+        const int r0 = t / TX * TR, c0 = t % TX * TC;
+#pragma unroll
+        for (int i = 0; i < TR; i++) {
+            float v[TC];
+            if constexpr (ADD) vld<float, TC>(v, D + (r0 + i) * LD + c0);
+#pragma unroll
+            for (int j = 0; j < TC; j++) {
+                const float x = NEG ? -acc[i][j] : acc[i][j];
+                v[j] = ADD ? v[j] + x : x;
+            }
+            vst<float, TC>(D + (r0 + i) * LD + c0, v);
+        }
+    }
+};
+
+template <int NT, int LD> struct BlkInv {
+    template <int N> static __device__ __forceinline__ bool run(float *S)
+    {
+        if constexpr (N == 32) {
+            bool ok = true;
+            if (threadIdx.x < 32) {
+                TileW<float, 32> t(threadIdx.x);
+                typename TileW<float, 32>::Reg x;
+#pragma unroll
+                for (int i = 0; i < t.TR; i++) t.ld_row(x[i], S + t.row(i) * LD);
+                ok = t.inverse(x);
+#pragma unroll
+                for (int i = 0; i < t.TR; i++) t.st_row(S + t.row(i) * LD, x[i]);
+            }
+            __syncthreads();
+            return ok;
+        } else {
+            // a product alone takes all threads (512 at most: 4 x 2 sub-tiles), two
+            // at once half of them each
+            constexpr int h = N / 2, N1 = NT > 512 ? 512 : NT, N2 = NT / 2;
+            using P1 = BlkMul<h, N1, LD>;
+            using P2 = BlkMul<h, N2, LD>;
+            float *A12 = S + h, *A21 = S + h * LD, *A22 = A21 + h;
+            const int t = threadIdx.x, t2 = t % N2;
+            const bool one = t < N1, lo = t < N2;
+            typename P1::Acc u;
+            typename P2::Acc v;
+            bool ok = run<h>(S); // H11
+            if (one) P1::mul(t, u, A21, S); // U = A21 H11
+            __syncthreads();
+            if (one) P1::template put<false, false>(t, A21, u);
+            __syncthreads();
+            P2::mul(t2, v, lo ? A21 : S, A12); // U A12; T = H11 A12
+            __syncthreads();
+            if (lo)
+                P2::template put<true, true>(t2, A22, v);
+            else
+                P2::template put<false, false>(t2, A12, v);
+            __syncthreads();
+            ok = run<h>(A22) && ok; // H22
+            P2::mul(t2, v, lo ? A12 : A22, lo ? A22 : A21); // T H22; H22 U
+            __syncthreads();
+            if (lo) P2::template put<false, true>(t2, A12, v); // G12
+            __syncthreads();
+            if (one) P1::mul(t, u, A12, A21); // G12 U
+            __syncthreads();
+            if (one) P1::template put<true, true>(t, S, u);     // G11
+            if (!lo) P2::template put<false, true>(t2, A21, v); // G21
+            __syncthreads();
+            return ok;
+        }
+    }
+};
+
+template <class T, int KB, int NT> __device__ __forceinline__ bool Tile<T, KB, NT>::inverse_blk(Reg &s, T *tile) const
+{
+    rstore(tile, s);
+    __syncthreads();
+    const bool ok = BlkInv<NT, LD>::template run<KB>(tile);
+    rload(s, tile);
+    return __syncthreads_and(ok ? 1 : 0) != 0;
+}
+template <class T, int KB> __device__ __forceinline__ bool Tile88<T, KB>::inverse_blk(Reg &s, T *tile) const
+{
+    rstore(tile, s);
+    __syncthreads();
+    const bool ok = BlkInv<NT, LD>::template run<KB>(tile);
+    rload(s, tile);
+    return __syncthreads_and(ok ? 1 : 0) != 0;
+}
 
 // Thread counts and tile geometry of the two-sided kernels: the elimination
 // chains of FP32 64-row tiles run on 64 threads with 8 x 8 sub-tiles (Tile88),

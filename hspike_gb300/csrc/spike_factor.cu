@@ -575,7 +575,10 @@ __global__ void __launch_bounds__(NTOf<KB>::value)
             cp_async_commit();
         }
         // G_J = S_J^{-1}
-        ok = t.inverse(acc, buf) && ok;
+        if constexpr (std::is_same<T, float>::value && KB == 64)
+            ok = t.inverse_blk(acc, sG) && ok; // (G_{J-1} is consumed)
+        else
+            ok = t.inverse(acc, buf) && ok;
         cp_async_wait_all();
         t.rstore(sG, acc);
         t.gstore_t(gG + tb + J * TS, acc); // column-major for the backward sweep

@@ -273,7 +273,12 @@ __global__ void __launch_bounds__(NTOf<KB>::value)
     tc_each<KB>(acc, [&](int r, int c, float v) { sH[r * LD + c] = (r == c ? 1.f : 0.f) - v; }); // S
     __syncthreads();
     t.rload(a, sH);
-    const bool ok = t.inverse(a, buf);
+    __syncthreads();
+    bool ok;
+    if constexpr (KB == 64)
+        ok = t.inverse_blk(a, sH);
+    else
+        ok = t.inverse(a, buf);
     if (!ok && threadIdx.x == 0) atomicOr(err, SPK_DEV_ERR_PIVOT);
     __syncthreads();
     t.rstore(sH, a); // M11

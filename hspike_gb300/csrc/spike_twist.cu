@@ -139,7 +139,10 @@ __global__ void __launch_bounds__(TwCfg<T, KB>::NT_LU, 4)
                     t.gload(dreg, gTp + (size_t)(J + 1) * 3 * TS); // D_{J+1}, lands during the inverse
                 }
             }
-            ok = t.inverse(acc, buf) && ok;
+            if constexpr (TwCfg<T, KB>::T88)
+                ok = t.inverse_blk(acc, buf) && ok;
+            else
+                ok = t.inverse(acc, buf) && ok;
             t.rstore(sG, acc);
             t.gstore_t(gG + tb + J * TS, acc);
             __syncthreads();
@@ -172,7 +175,10 @@ __global__ void __launch_bounds__(TwCfg<T, KB>::NT_LU, 4)
                 b2.issue_dense<T, KB>(sX, gTp + (size_t)J * 3 * TS + TS);
                 t.gload(dreg, gTp + (size_t)(J - 1) * 3 * TS); // D_{J-1}
             }
-            ok = t.inverse(acc, buf) && ok;
+            if constexpr (TwCfg<T, KB>::T88)
+                ok = t.inverse_blk(acc, buf) && ok;
+            else
+                ok = t.inverse(acc, buf) && ok;
             t.rstore(sH, acc);
             t.gstore_t(gG + tb + J * TS, acc);
             __syncthreads();
@@ -668,7 +674,11 @@ __global__ void __launch_bounds__(TwCfg<T, KB>::NT_LU, 4)
     __syncthreads();
     t.gload(acc, gG + tb + M * TS); // T'_M
     t.mms_t_bl(acc, sC, sB);        // S_M = T'_M - L_M A(M-1,M) (lower triangular)
-    const bool ok = t.inverse(acc, buf);
+    bool ok;
+    if constexpr (TwCfg<T, KB>::T88)
+        ok = t.inverse_blk(acc, buf);
+    else
+        ok = t.inverse(acc, buf);
     t.rstore_t(sA, acc); // G_M as a left operand
     t.gstore_t(gG + tb + M * TS, acc);
     __syncthreads();
