@@ -1179,6 +1179,8 @@ template <class T, int KB> int run_factor(spk_plan *P, const int *rowptr, const 
     using H = typename HighOf<T>::type;
     constexpr int NT = NTOf<KB>::value;
     using S = FactorSmem<T, KB>;
+    // 64-row FP64 tiles: the chains' products on the tensor cores
+    constexpr bool EMU = std::is_same<T, double>::value && KB == 64;
     static bool attr = false;
     if (!attr) {
         if constexpr (S::BIG) {
@@ -1199,13 +1201,16 @@ template <class T, int KB> int run_factor(spk_plan *P, const int *rowptr, const 
                                      (int)QuadBwd<T, KB>::SMEM) != cudaSuccess)
                 return SPK_ECUDA;
         }
-        if (cudaFuncSetAttribute(k_factor_fwd<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::fwd) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(k_band_tiles<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::band) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(k_factor_bwd<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bwd) !=
-                cudaSuccess)
+        if (cudaFuncSetAttribute(k_band_tiles<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::band) !=
+            cudaSuccess)
             return SPK_ECUDA;
+        if constexpr (!EMU) {
+            if (cudaFuncSetAttribute(k_factor_fwd<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::fwd) !=
+                    cudaSuccess ||
+                cudaFuncSetAttribute(k_factor_bwd<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bwd) !=
+                    cudaSuccess)
+                return SPK_ECUDA;
+        }
         }
         attr = true;
     }
@@ -1242,6 +1247,8 @@ template <class T, int KB> int run_factor(spk_plan *P, const int *rowptr, const 
         const int cpc = chains_per_cta(P->p, CF::CPC);
         k_quad_fwd<T, KB><<<(P->p + cpc - 1) / cpc, cpc * KB, (size_t)cpc * CF::SLOT, st>>>(
             (const T *)P->d_T, P->d_blk_off, P->p, (T *)P->d_L, (T *)P->d_G, (T *)P->d_W, P->d_err);
+    } else if constexpr (EMU) {
+        if (const int rc_ = spk_emu_factor(P, 1, st); rc_ != SPK_OK) return rc_;
     } else {
         k_factor_fwd<T, KB><<<P->p, NT, S::fwd, st>>>((const T *)P->d_T, P->d_blk_off, (T *)P->d_L, (T *)P->d_G,
                                                       (T *)P->d_W, P->d_err);
@@ -1261,6 +1268,8 @@ template <class T, int KB> int run_factor(spk_plan *P, const int *rowptr, const 
             k_quad_bwd<T, KB><<<(2 * P->p + cpc - 1) / cpc, cpc * KB, (size_t)cpc * CB::SLOT, st>>>(
                 P->d_part_start, P->d_blk_off, P->p, (const T *)P->d_L, (const T *)P->d_G, (const T *)P->d_E,
                 (const T *)P->d_W, (const T *)P->d_Bhat, (T *)P->d_V, (T *)P->d_W);
+        } else if constexpr (EMU) {
+            if (const int rc_ = spk_emu_factor(P, 0, st); rc_ != SPK_OK) return rc_;
         } else {
             k_factor_bwd<T, KB><<<P->p, NT, S::bwd, st>>>(P->d_part_start, P->d_blk_off, P->p, (const T *)P->d_L,
                                                           (const T *)P->d_G, (const T *)P->d_E, (T *)P->d_W,

@@ -269,6 +269,15 @@ int spk_factor_range(spk_plan *P, const int *d_rowptr, const int *d_colind, cons
                      void *stream);
 int spk_factor_tips(spk_plan *P, void *stream);
 
+/* ---- 64-row FP64 tiles, products on the tensor cores (spike_emu64.cu) ---- */
+/* the one-sided chains: forward = 1: block LU and W's sweep; 0: the spikes */
+int spk_emu_factor(spk_plan *P, int forward, void *stream);
+/* the reduced system's cyclic reduction: odd blocks, even blocks */
+int spk_emu_cr_odd(const double *P, const double *Q, int first, int stride, int count, double *M, unsigned *err,
+                   void *stream);
+int spk_emu_cr_even(const double *P, const double *Q, const double *X, const double *Y, const double *M, int cnt,
+                    double *Pn, double *Qn, double *Xn, double *Yn, void *stream);
+
 /* ---- reduced system (spike_reduced.cu) ---- */
 int spk_reduced_factor(spk_plan *P, void *stream);
 /* u = R^{-1} g for nrhs columns (FP64), with refine_iters FP64 refinement

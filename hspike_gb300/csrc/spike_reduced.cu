@@ -557,11 +557,17 @@ template <class T, int KB> int run_red_factor(spk_plan *P, cudaStream_t st)
     } else {
     // FP32 factors with 64- or 128-row tiles: the block products on the tensor cores
     constexpr bool TC = std::is_same<T, float>::value && (KB == 64 || KB == 128);
+    // FP64 with 64-row tiles: likewise, by exact digit products (spike_emu64.cu)
+    constexpr bool EMU = std::is_same<T, double>::value && KB == 64;
     static bool attr = false;
     if (!attr) {
-        if (cudaFuncSetAttribute(k_cr_odd<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes) != cudaSuccess ||
-            cudaFuncSetAttribute(k_cr_even<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes) != cudaSuccess)
-            return SPK_ECUDA;
+        if constexpr (!TC && !EMU) {
+            if (cudaFuncSetAttribute(k_cr_odd<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes) !=
+                    cudaSuccess ||
+                cudaFuncSetAttribute(k_cr_even<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes) !=
+                    cudaSuccess)
+                return SPK_ECUDA;
+        }
         if constexpr (TC) {
             if (cudaFuncSetAttribute(k_cr_odd_tc<KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes) !=
                     cudaSuccess ||
@@ -572,7 +578,9 @@ template <class T, int KB> int run_red_factor(spk_plan *P, cudaStream_t st)
         attr = true;
     }
     auto odd = [&](const T *Pp, const T *Qp, int first, int stride, int count, T *Mo) {
-        if constexpr (TC)
+        if constexpr (EMU)
+            spk_emu_cr_odd(Pp, Qp, first, stride, count, Mo, P->d_err, st);
+        else if constexpr (TC)
             k_cr_odd_tc<KB><<<count, NT, S::bytes, st>>>(Pp, Qp, first, stride, Mo, P->d_err);
         else
             k_cr_odd<T, KB><<<count, NT, S::bytes, st>>>(Pp, Qp, first, stride, Mo, P->d_err);
@@ -587,7 +595,9 @@ template <class T, int KB> int run_red_factor(spk_plan *P, cudaStream_t st)
             odd(cP + o, cQ + o, 1, 2, nodd, Ml);
             SPK_CHECK_LAUNCH();
         }
-        if constexpr (TC)
+        if constexpr (EMU)
+            spk_emu_cr_even(cP + o, cQ + o, cX + o, cY + o, Ml, cnt, cP + on, cQ + on, cX + on, cY + on, st);
+        else if constexpr (TC)
             k_cr_even_tc<KB><<<dim3(neven, 4), NT, S::bytes, st>>>(cP + o, cQ + o, cX + o, cY + o, Ml, cnt, cP + on,
                                                                    cQ + on, cX + on, cY + on);
         else

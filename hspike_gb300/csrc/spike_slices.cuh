@@ -111,15 +111,15 @@ struct SlAcc {
         }
     }
     // += the step's products; bfrag(i, r): register r of digit i's right
-    // fragment (i = SL_D: the magnitudes')
-    template <class B> __device__ __forceinline__ void step(const SlFragA &A, B bfrag)
+    // fragment (i = SL_D: the magnitudes').  ND < SL_D: the leading ND sums only.
+    template <int ND = SL_D, class B> __device__ __forceinline__ void step(const SlFragA &A, B bfrag)
     {
         sl_mma(g, A.mg, bfrag(SL_D, 0), bfrag(SL_D, 1));
 #pragma unroll
-        for (int j = 0; j < SL_D; j++) {
+        for (int j = 0; j < ND; j++) {
             const unsigned b0 = bfrag(j, 0), b1 = bfrag(j, 1);
 #pragma unroll
-            for (int i = 0; i + j < SL_D; i++) sl_mma(c[i + j], A.a[i], b0, b1);
+            for (int i = 0; i + j < ND; i++) sl_mma(c[i + j], A.a[i], b0, b1);
         }
     }
     // element e as integers, hi 2^32 + lo in units of 256^7
@@ -142,24 +142,22 @@ __device__ __forceinline__ double sl_round(long long hi, long long lo, int p)
 {
     hi += lo >> 32;
     unsigned w0 = (unsigned)lo; // value = hi 2^32 + w0
-    const unsigned neg = hi < 0 ? 0xffffffffu : 0u;
-    if (neg) {
-        w0 = 0u - w0;
-        hi = ~hi + (w0 == 0u ? 1 : 0);
-    }
-    unsigned long long h = (unsigned long long)hi;
-    if (h == 0) {
-        if (w0 == 0u) return 0.0;
-        h = (unsigned long long)w0 << 31;
-        w0 = 0u;
-        p -= 63;
-    }
-    const int z = __clzll((long long)h);
-    unsigned long long m = (h << z) | (z ? ((unsigned long long)w0 << 32) >> (64 - z) : 0ull); // top bit at 63
+    const unsigned neg = (unsigned)((int)(hi >> 32) >> 31);
+    // (no branches: several results are in flight at once)
+    w0 = (w0 ^ neg) - neg;
+    unsigned long long h = ((unsigned long long)hi ^ (((unsigned long long)neg << 32) | neg)) + (neg && w0 == 0u ? 1u : 0u);
+    const bool small = h == 0;
+    h = small ? (unsigned long long)w0 << 31 : h;
+    p = small ? p - 63 : p;
+    const unsigned wl = small ? 0u : w0;
+    const bool none = h == 0;
+    const int z = __clzll((long long)h) & 63; // h < 2^62 unless small (bit 63 free)
+    unsigned long long m = (h << z) | (((unsigned long long)wl << 31) >> (63 - z)); // top bit at 63
     p += 32 - z;
-    const unsigned long long rest = m & 0x7ffull;
-    unsigned long long f = (m >> 11) + (rest > 0x400ull || (rest == 0x400ull && ((m >> 11) & 1)) ? 1 : 0); // 53 bits
-    // f 2^(p + 11): a carry to 2^53 bumps the exponent through the addition
-    const unsigned long long bits = ((unsigned long long)(p + 11 + 52 + 1022) << 52) + f;
-    return __longlong_as_double((long long)(bits | ((unsigned long long)(neg & 0x80000000u) << 32)));
+    const unsigned rest = (unsigned)m & 0x7ffu;
+    m >>= 11;
+    m += rest > 0x400u || (rest == 0x400u && ((unsigned)m & 1u)) ? 1u : 0u; // 53 bits, to nearest
+    // m 2^(p + 11): a carry to 2^53 bumps the exponent through the addition
+    const unsigned long long bits = ((unsigned long long)(unsigned)(p + 11 + 52 + 1022) << 52) + m;
+    return none ? 0.0 : __longlong_as_double((long long)(bits | ((unsigned long long)(neg & 0x80000000u) << 32)));
 }
