@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(256)
             const long long row = base + lane / G;
             const bool valid = row < n;
             const int t0 = valid ? rowptr[row] : 0, t1 = valid ? rowptr[row + 1] : 0;
-            // IMPL: the row is the full band (checked on the host), colind is not read
+            // IMPL: the row is the full band, colind is not read
             const int cfirst = IMPL ? max(0, (int)row - impl_kl) - t0 : 0;
             H acc[NH];
 #pragma unroll
@@ -383,6 +383,24 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// every row holds all of its band's columns: distinct columns within ku, kl,
+// and as many as there can be
+static bool full_band(const spk_plan *P)
+{
+    const long long ku = P->ku < P->n - 1 ? P->ku : P->n - 1, kl = P->kl < P->n - 1 ? P->kl : P->n - 1;
+    return P->nnz == P->n * (ku + kl + 1) - (ku * (ku + 1) + kl * (kl + 1)) / 2;
+}
+
+// the band's lower width where the rows' columns follow from the row pointers
+// alone, so that colind, a third of the matrix's bytes, need not be read; else
+// -1.  One column: n = 300,000, k = 8 34 -> 31 us; n = 2,000,000, k = 64 608 ->
+// 587 us, where the FP64 pipe takes over.
+static int implied_kl(const spk_plan *P)
+{
+    if (P->impl_cols) return P->impl_kl;
+    return full_band(P) ? P->kl : -1;
+}
+
 template <class H, int G, bool IMPL>
 static int launch_residual(const spk_plan *P, const int *rp, const int *ci, const void *a, const void *x, const void *b,
                            void *r, int nrhs, int want_b, double *norms, cudaStream_t st)
@@ -395,15 +413,15 @@ static int launch_residual(const spk_plan *P, const int *rp, const int *ci, cons
         if (nr >= 4)
             k_residual<H, G, 4, IMPL><<<(unsigned)blocks, 256, 0, st>>>(P->n, rp, ci, (const H *)a, (const H *)x,
                                                                  (const H *)b, (H *)r, h0, nr, want_b, norms, nrhs,
-                                                                 P->impl_cols ? P->impl_kl : -1);
+                                                                 implied_kl(P));
         else if (nr >= 2)
             k_residual<H, G, 2, IMPL><<<(unsigned)blocks, 256, 0, st>>>(P->n, rp, ci, (const H *)a, (const H *)x,
                                                                  (const H *)b, (H *)r, h0, nr, want_b, norms, nrhs,
-                                                                 P->impl_cols ? P->impl_kl : -1);
+                                                                 implied_kl(P));
         else
             k_residual<H, G, 1, IMPL><<<(unsigned)blocks, 256, 0, st>>>(P->n, rp, ci, (const H *)a, (const H *)x,
                                                                  (const H *)b, (H *)r, h0, nr, want_b, norms, nrhs,
-                                                                 P->impl_cols ? P->impl_kl : -1);
+                                                                 implied_kl(P));
         if (cudaGetLastError() != cudaSuccess) return SPK_ECUDA;
         ((spk_plan *)P)->launches++;
     }
@@ -428,7 +446,7 @@ static int residual_g(const spk_plan *P, const int *rp, const int *ci, const voi
     // one column: 4 lanes from 64 entries a row; several columns: 2 lanes (a
     // lane's multiply-adds per reduction step grow with the columns)
     const int g = res_lanes(per_row, nrhs);
-    if (P->impl_cols) {
+    if (implied_kl(P) >= 0) {
         if (g == 4) return launch_residual<H, 4, true>(P, rp, ci, a, x, b, r, nrhs, want_b, norms, st);
         if (g == 2) return launch_residual<H, 2, true>(P, rp, ci, a, x, b, r, nrhs, want_b, norms, st);
         return launch_residual<H, 1, true>(P, rp, ci, a, x, b, r, nrhs, want_b, norms, st);
@@ -436,14 +454,6 @@ static int residual_g(const spk_plan *P, const int *rp, const int *ci, const voi
     if (g == 4) return launch_residual<H, 4, false>(P, rp, ci, a, x, b, r, nrhs, want_b, norms, st);
     if (g == 2) return launch_residual<H, 2, false>(P, rp, ci, a, x, b, r, nrhs, want_b, norms, st);
     return launch_residual<H, 1, false>(P, rp, ci, a, x, b, r, nrhs, want_b, norms, st);
-}
-
-// every row holds all of its band's columns: distinct columns within ku, kl,
-// and as many as there can be
-static bool full_band(const spk_plan *P)
-{
-    const long long ku = P->ku < P->n - 1 ? P->ku : P->n - 1, kl = P->kl < P->n - 1 ? P->kl : P->n - 1;
-    return P->nnz == P->n * (ku + kl + 1) - (ku * (ku + 1) + kl * (kl + 1)) / 2;
 }
 
 extern "C" int spk_residual(const spk_plan *P, const int *d_rowptr, const int *d_colind, const void *d_aij,
