@@ -1510,16 +1510,23 @@ template <class T, int KB, int NT> __device__ __forceinline__ void cp_async_tile
 // if-converted hardware conversion would run on the FP64 pipe for every value.
 static __device__ __noinline__ float f64_to_f32_rare(double x) { return (float)x; }
 static __device__ __noinline__ double f32_to_f64_rare(float x) { return (double)x; }
-__device__ __forceinline__ float f64_to_f32(double x)
+// (rare is set, and the result meaningless, where the hardware has to convert)
+__device__ __forceinline__ float f64_to_f32_try(double x, bool &rare)
 {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    const int e = (int)((hi >> 20) & 0x7ffu) - 1023 + 127;
-    if (e <= 0 || e >= 255) return f64_to_f32_rare(x);
-    const unsigned r = ((hi & 0xfffffu) << 3) | (lo >> 29); // 23 mantissa bits
-    const unsigned rem = lo & 0x1fffffffu;                  // 29 dropped bits
-    const unsigned up = (rem > 0x10000000u) || (rem == 0x10000000u && (r & 1u));
-    // a carry out of the mantissa bumps the exponent (to inf at the top), as it should
-    return __uint_as_float(((hi & 0x80000000u) | ((unsigned)e << 23)) + r + up);
+    rare = rare || ((hi >> 20) & 0x7ffu) - 897u >= 254u; // FP32 exponents 1 to 254 only
+    // the 29 dropped bits round to nearest even; a carry out of the mantissa
+    // bumps the exponent (to inf at the top), as it should
+    const unsigned long long r = (((unsigned long long)hi << 32) | lo) + (0x0fffffffu + ((lo >> 29) & 1u));
+    // exponent from bias 1023 to 127: its two top bits leave, 896 = 0x180 modulo 512 with them
+    const unsigned f = __funnelshift_l((unsigned)r, (unsigned)(r >> 32), 3) - 0xc0000000u;
+    return __uint_as_float((hi & 0x80000000u) | f);
+}
+__device__ __forceinline__ float f64_to_f32(double x)
+{
+    bool rare = false;
+    const float f = f64_to_f32_try(x, rare);
+    return rare ? f64_to_f32_rare(x) : f;
 }
 // FP32 -> FP64 (exact) with integer instructions, for the same reason.  Normal
 // inputs only; zero, subnormal, inf and NaN take the hardware conversion.
@@ -1541,6 +1548,14 @@ template <> __device__ __forceinline__ float cvt_fast<float, double>(double v) {
 template <> __device__ __forceinline__ cfloat cvt_fast<cfloat, cdouble>(cdouble v)
 {
     return {f64_to_f32(v.re), f64_to_f32(v.im)};
+}
+
+// cvt_fast without its branch: several conversions share one
+template <class T, class H> __device__ __forceinline__ T cvt_try(H v, bool &) { return sc_cvt<T, H>(v); }
+template <> __device__ __forceinline__ float cvt_try<float, double>(double v, bool &rare) { return f64_to_f32_try(v, rare); }
+template <> __device__ __forceinline__ cfloat cvt_try<cfloat, cdouble>(cdouble v, bool &rare)
+{
+    return {f64_to_f32_try(v.re, rare), f64_to_f32_try(v.im, rare)};
 }
 
 // ------------------------------------------------------------ warp sums

@@ -39,23 +39,28 @@ template <class T, int KB> struct FactorSmem {
     // k_band_tiles: small tiles pack BG row blocks into one CTA (one warp or
     // warp pair each), so the grid is not a million one-warp CTAs
     static constexpr int BG = KB <= 16 ? 256 / NTOf<KB>::value : 1;
+    // resident CTAs: 64-row tiles have 80 registers a thread for two batches of entries
+    static constexpr int BAND_CTAS = KB >= 128 ? 1 : KB == 64 ? (sizeof(T) == 4 ? 3 : 2) : KB == 32 ? 8 : 4;
     static constexpr size_t band_one = (3 * sizeof(T) * KB * (KB + 1) + sizeof(int) * (KB + 1) + 15) / 16 * 16;
     static constexpr size_t band = BG * band_one + 64;
     static constexpr size_t bwd = (BIG ? 3 : 6) * tile + 64; // (also k_wsweep_big: three tiles)
 };
 
-// Scatter the CSR rows of block J of partition [s, e) into the shared tiles.
-// F: columns of block J-1 (stored transposed: it is the left operand of
-// F G), D: block J, En: block J+1 (shared tiles, row stride LD); gZ (global,
-// row-major, zeroed by the caller): C^ coupling (J == 0, columns s-KB..s-1);
-// gBhat (global, row-major): B^ coupling (columns e..e+KB-1).
-// One warp per row: the row's entries are contiguous, so the loads are
-// coalesced and every entry's row is known without a search; up to five
-// 32-entry chunks of a row (a whole row of a 64-row tile's band) are in
-// flight per iteration.
-template <class T, class H, int KB, int LD>
-__device__ __forceinline__ void place_entry(int lr, int lrow, int c, H a, int s, int m, int J, T *F, T *D, T *En,
-                                            T *gZ, T *gBhat, unsigned *err)
+// Scatter the CSR rows of block J of partition [s, e) into the shared image W
+// of the block row: row-major with row stride BandW<KB>::LD, columns of block
+// J-1, J and J+1 side by side, so that an entry's place is its row's start plus
+// its column.  gZ (global, row-major, zeroed by the caller): C^ coupling
+// (J == 0, columns s-KB..s-1); gBhat (global, row-major): B^ coupling (columns
+// e..e+KB-1).  One warp per row: the row's entries are contiguous, so the loads
+// are coalesced and every entry's row is known without a search; up to five
+// 32-entry chunks of a row (a whole row of a 64-row tile's band) are in flight
+// per iteration.
+template <int KB> struct BandW {
+    static constexpr int LD = 3 * KB + 1; // odd: conflict-free for row-major and column-major reads
+};
+template <class T, class H, int KB>
+__device__ __forceinline__ void place_entry(int lr, int lrow, int c, H a, int s, int m, int J, T *W, T *gZ, T *gBhat,
+                                            unsigned *err)
 {
     const T v = cvt_fast<T, H>(a);
     const int lc = c - s;
@@ -72,14 +77,9 @@ __device__ __forceinline__ void place_entry(int lr, int lrow, int c, H a, int s,
         } else
             atomicOr(err, SPK_DEV_ERR_BAND);
     } else {
-        const int bc = lc / KB, cc = lc - bc * KB;
-        const int d = bc - J;
-        if (d == 0)
-            D[lr * LD + cc] = v;
-        else if (d == -1)
-            F[cc * LD + lr] = v;
-        else if (d == 1)
-            En[lr * LD + cc] = v;
+        const int rel = lc - (J - 1) * KB;
+        if ((unsigned)rel < 3u * KB)
+            W[lr * BandW<KB>::LD + rel] = v;
         else
             atomicOr(err, SPK_DEV_ERR_BAND);
     }
@@ -92,32 +92,46 @@ __device__ __forceinline__ void place_entry(int lr, int lrow, int c, H a, int s,
 // pointers is flagged and not read.  impl_kl >= 0: colind is not read; the
 // host verified that every row is the full band, so entry t of row r is
 // column max(0, r - impl_kl) + (t - rowptr[r]).
-template <class T, class H, int KB, int LD, bool VAL, bool IMPL = false>
+template <class T, class H, int KB, bool VAL, bool IMPL = false>
 __device__ __forceinline__ void scatter_block(const int *__restrict__ rowptr, const int *__restrict__ colind,
-                              const H *__restrict__ aij, int s, int e, int J, T *F, T *D, T *En, T *gZ,
+                              const H *__restrict__ aij, int s, int e, int J, T *W, T *gZ,
                               T *gBhat, unsigned *err, int *srp, int n, long long nnz, int impl_kl, int tid,
                               bool live)
 {
-    constexpr int NT = NTOf<KB>::value;
+    constexpr int NT = NTOf<KB>::value, LD = BandW<KB>::LD;
     constexpr int NW = NT / 32;
     const int m = e - s;
     const int lrow0 = J * KB;
     const int nr = min(KB, m - lrow0); // real rows in the block, >= 1
     if (live) {
         for (int q = tid; q <= nr; q += NT) srp[q] = rowptr[s + lrow0 + q];
-        for (int lr = nr + tid; lr < KB; lr += NT) D[lr * LD + lr] = sc_one<T>(); // identity padding
+        for (int lr = nr + tid; lr < KB; lr += NT) W[lr * LD + KB + lr] = sc_one<T>(); // identity padding
     }
     __syncthreads();
     if (!live) return; // (a CTA's spare block slot: every barrier above is shared)
     const int warp = tid >> 5, lane = tid & 31;
+    // all three block columns lie inside the partition: an entry is in them or outside the band
+    const bool inner = J > 0 && (long long)(J + 2) * KB <= m;
+    const int w0 = s + (J - 1) * KB; // the image's first column
+    auto place = [&](int lr, int c, H a) {
+        if (inner) {
+            if ((unsigned)(c - w0) < 3u * KB)
+                W[lr * LD + (c - w0)] = cvt_fast<T, H>(a);
+            else
+                atomicOr(err, SPK_DEV_ERR_BAND);
+        } else {
+            place_entry<T, H, KB>(lr, lrow0 + lr, c, a, s, m, J, W, gZ, gBhat, err);
+        }
+    };
     // pieces per iteration: a whole row of the band (2 KB + 1 entries) in one go
     constexpr int PPR = (2 * KB + 1 + 31) / 32 < 1 ? 1 : (2 * KB + 1 + 31) / 32 > 5 ? 5 : (2 * KB + 1 + 31) / 32;
     int ku = 0, kl = 0;
     if constexpr (KB <= 16) {
         // Short rows (2 KB + 1 <= 33 entries): the block's entries are one
         // contiguous run, so the threads take it flat -- every entry of every
-        // row in flight at once -- and find each entry's row among the block's
-        // row pointers in shared memory.
+        // row in flight at once -- and find each entry's row by a division
+        // where all rows are as long as the first (inside a full band), else
+        // among the block's row pointers in shared memory.
         const int T0 = srp[0], T1 = srp[nr];
         bool rows_ok = T0 >= 0 && (long long)T1 <= nnz && T1 >= T0;
         if constexpr (VAL) {
@@ -125,6 +139,11 @@ __device__ __forceinline__ void scatter_block(const int *__restrict__ rowptr, co
                 if (srp[q] < 0 || (long long)srp[q + 1] > nnz || srp[q + 1] < srp[q]) atomicOr(err, SPK_DEV_ERR_CSR);
             if (!rows_ok && tid == 0) atomicOr(err, SPK_DEV_ERR_CSR);
         }
+        const int len = srp[1] - T0;
+        bool same = rows_ok && len >= 2 && len <= 2 * KB + 1;
+#pragma unroll
+        for (int q = 2; q <= KB; q++) same = same && (q > nr || srp[q] - T0 == q * len);
+        const unsigned inv = same ? 0xffffffffu / (unsigned)len + 1u : 0u; // floor(x / len) = x inv >> 32 for x < 2^16
         constexpr int U = 4; // entries per thread in flight
         for (int base = rows_ok ? T0 : T1; base < T1; base += NT * U) {
             int c[U], lrs[U];
@@ -135,8 +154,12 @@ __device__ __forceinline__ void scatter_block(const int *__restrict__ rowptr, co
                 lrs[u] = 0;
                 if (t < T1) {
                     int lr = 0;
+                    if (same) {
+                        lr = (int)__umulhi((unsigned)(t - T0), inv);
+                    } else {
 #pragma unroll
-                    for (int q = 1; q < KB; q++) lr += (q < nr && srp[q] <= t);
+                        for (int q = 1; q < KB; q++) lr += (q < nr && srp[q] <= t);
+                    }
                     lrs[u] = lr;
                     c[u] = IMPL ? max(0, s + lrow0 + lr - impl_kl) + (t - srp[lr]) : __ldg(colind + t);
                     a[u] = aij[t];
@@ -153,12 +176,75 @@ __device__ __forceinline__ void scatter_block(const int *__restrict__ rowptr, co
                         ku = max(ku, c[u] - grow);
                         kl = max(kl, grow - c[u]);
                     }
-                    place_entry<T, H, KB, LD>(lr, lrow0 + lr, c[u], a[u], s, m, J, F, D, En, gZ, gBhat, err);
+                    place(lr, c[u], a[u]);
                 }
             }
         }
-    } else
-    for (int lr = warp; lr < nr; lr += NW) {
+    } else {
+    // Inside a full band every row has the same L columns one further right:
+    // the block's entries are one run whose place in the image follows from
+    // their index, and the columns are only compared with what they must be
+    // (where one differs the block starts again below).  n = 2,000,000, k = 64:
+    // 1,238 us row by row into three tiles (81 instructions per 32 entries),
+    // 1,004 row by row into the image, 880 so, 5.3 TB/s of reads and writes.
+    bool done = false;
+    {
+        const int T0 = srp[0], L = srp[1] - T0, f0 = IMPL ? s + lrow0 - impl_kl : T0 >= 0 && T0 < nnz ? __ldg(colind + T0) : -1;
+        bool flat = inner && nr == KB && L >= 2 && L <= 2 * KB + 1 && T0 >= 0 && (long long)T0 + KB * L <= nnz &&
+                    f0 >= w0 && f0 - w0 <= 3 * KB - (KB + L - 1);
+        // the entries come in batches of U per thread, each on its way while the
+        // one before is placed, the first before the barrier
+        constexpr int U = (KB == 64 ? 6 : 4) * 8 / (int)sizeof(H);
+        int c[2][U];
+        H a[2][U];
+        auto fetch = [&](int x0, int (&cc)[U], H (&aa)[U]) {
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (x0 + u * NT < KB * L) {
+                    if constexpr (!IMPL) cc[u] = __ldg(colind + T0 + x0 + u * NT);
+                    aa[u] = aij[T0 + x0 + u * NT];
+                }
+        };
+        if (flat) fetch(tid, c[0], a[0]);
+        for (int q = tid; flat && q <= KB; q += NT) flat = srp[q] == T0 + q * L;
+        if (__syncthreads_and(flat)) {
+            const unsigned inv = 0xffffffffu / (unsigned)L + 1u; // floor(x / L) = x inv >> 32 for x < 2^16
+            T *w = W + (f0 - w0);
+            bool ok = true;
+            auto put = [&](int x0, const int (&cc)[U], const H (&aa)[U]) {
+                bool rare = false; // zeros, say: converted again
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (x0 + u * NT < KB * L) {
+                        const int x = x0 + u * NT, lr = (int)__umulhi((unsigned)x, inv);
+                        if constexpr (!IMPL) ok = ok && cc[u] == f0 + x - lr * (L - 1);
+                        w[x + lr * (LD + 1 - L)] = cvt_try<T, H>(aa[u], rare);
+                    }
+                if (rare)
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (x0 + u * NT < KB * L) {
+                            const int x = x0 + u * NT, lr = (int)__umulhi((unsigned)x, inv);
+                            w[x + lr * (LD + 1 - L)] = cvt_fast<T, H>(aa[u]);
+                        }
+            };
+            for (int base = tid; base < KB * L; base += 2 * NT * U) {
+                fetch(base + NT * U, c[1], a[1]);
+                put(base, c[0], a[0]);
+                fetch(base + 2 * NT * U, c[0], a[0]);
+                put(base + NT * U, c[1], a[1]);
+            }
+            done = IMPL || __syncthreads_and(ok);
+            if (done) {
+                ku = f0 + L - 1 - (s + lrow0);
+                kl = s + lrow0 - f0;
+            } else {
+                for (int q = tid; q < KB * LD; q += NT) W[q] = sc_zero<T>();
+                __syncthreads();
+            }
+        }
+    }
+    for (int lr = done ? nr : warp; lr < nr; lr += NW) {
         const int t0 = srp[lr], t1 = srp[lr + 1];
         if (VAL && (t0 < 0 || (long long)t1 > nnz || t1 < t0)) {
             if (lane == 0) atomicOr(err, SPK_DEV_ERR_CSR);
@@ -194,9 +280,9 @@ __device__ __forceinline__ void scatter_block(const int *__restrict__ rowptr, co
             }
 #pragma unroll
             for (int u = 0; u < PPR; u++)
-                if (t + 32 * u < t1)
-                    place_entry<T, H, KB, LD>(lr, lrow0 + lr, c[u], a[u], s, m, J, F, D, En, gZ, gBhat, err);
+                if (t + 32 * u < t1) place(lr, c[u], a[u]);
         }
+    }
     }
     if constexpr (VAL) {
         for (int o = 16; o > 0; o >>= 1) {
@@ -255,7 +341,7 @@ __device__ __forceinline__ void store_tile_cm(T *g, const T *s)
 // bottom-up chain instead (spike_twist.cu): A(J,J-1) row-major in gT and
 // column-major in gE for J > M, A(J,J+1) column-major in gT for J >= M.
 template <class T, int KB>
-__global__ void __launch_bounds__(NTOf<KB>::value * FactorSmem<T, KB>::BG)
+__global__ void __launch_bounds__(NTOf<KB>::value * FactorSmem<T, KB>::BG, FactorSmem<T, KB>::BAND_CTAS)
     k_band_tiles(const int *__restrict__ rowptr, const int *__restrict__ colind,
                  const typename HighOf<T>::type *__restrict__ aij, const int *__restrict__ part_start,
                  const int *__restrict__ blk_off, const int *__restrict__ blk_part, T *gT, T *gE, T *gZ, T *gBhat,
@@ -284,47 +370,55 @@ __global__ void __launch_bounds__(NTOf<KB>::value * FactorSmem<T, KB>::BG)
         e -= (int)S.row0;
     }
 
-    // odd row stride: conflict-free for the row-major and the column-major stores
-    constexpr int LD1 = KB + 1;
-    constexpr int EL1 = KB * LD1;
+    constexpr int LD = BandW<KB>::LD, EL = KB * LD; // the image of the block row
     extern __shared__ char smraw[];
-    T *sD = (T *)(smem_align(smraw) + grp * FS::band_one), *sF = sD + EL1, *sE = sF + EL1;
-    int *srp = (int *)(sE + EL1);
+    T *W = (T *)(smem_align(smraw) + grp * FS::band_one);
+    int *srp = (int *)(W + EL);
     T *gz = zt ? gZ + (size_t)blk_off[part] * TS : nullptr;
-    for (int q = tid; q < 3 * EL1; q += NT) sD[q] = sc_zero<T>(); // sD, sF, sE are consecutive
+    if constexpr (EL * sizeof(T) % 16 == 0)
+        for (int q = tid; q < (int)(EL * sizeof(T) / 16); q += NT) ((uint4 *)W)[q] = make_uint4(0, 0, 0, 0);
+    else
+        for (int q = tid; q < EL; q += NT) W[q] = sc_zero<T>();
     if (zt)
         for (int q = tid; q < KB * KB; q += NT) gz[q] = sc_zero<T>();
     __syncthreads();
     if (validate) {
-        scatter_block<T, H, KB, LD1, true>(rowptr, colind, aij, s, e, J, sF, sD, sE, gz, gBhat + (size_t)part * TS,
-                                           err, srp, n, nnz, impl_kl, tid, live);
+        scatter_block<T, H, KB, true>(rowptr, colind, aij, s, e, J, W, gz, gBhat + (size_t)part * TS, err, srp, n, nnz,
+                                      impl_kl, tid, live);
         if (live && tid == 0 && ((gb == 0 && rowptr[0] != 0) || (gb == nb_total - 1 && (long long)rowptr[n] != nnz)))
             atomicOr(err, SPK_DEV_ERR_CSR);
     } else if (impl_kl >= 0) {
-        scatter_block<T, H, KB, LD1, false, true>(rowptr, colind, aij, s, e, J, sF, sD, sE, gz,
-                                                  gBhat + (size_t)part * TS, err, srp, n, nnz, impl_kl, tid, live);
+        scatter_block<T, H, KB, false, true>(rowptr, colind, aij, s, e, J, W, gz, gBhat + (size_t)part * TS, err, srp, n,
+                                             nnz, impl_kl, tid, live);
     } else {
-        scatter_block<T, H, KB, LD1, false>(rowptr, colind, aij, s, e, J, sF, sD, sE, gz, gBhat + (size_t)part * TS,
-                                            err, srp, n, nnz, impl_kl, tid, live);
+        scatter_block<T, H, KB, false>(rowptr, colind, aij, s, e, J, W, gz, gBhat + (size_t)part * TS, err, srp, n, nnz,
+                                       impl_kl, tid, live);
     }
     __syncthreads();
     if (!live) return;
-    // shared tile (row stride LD1) -> global tile, row-major or column-major
-    auto put = [&](T *g, const T *sm, bool cm) {
-        for (int q = tid; q < KB * KB; q += NT) {
-            const int a = q / KB, b = q - a * KB;
-            g[q] = cm ? sm[b * LD1 + a] : sm[a * LD1 + b];
+    // block column d (0: J-1, 1: J, 2: J+1) of the image -> global tile, row-major or column-major
+    auto put = [&](T *g, int d, bool cm) {
+        const T *w = W + d * KB;
+        const int a0 = tid / KB, b = tid % KB; // NT is a multiple of KB
+        if (cm) {
+#pragma unroll
+            for (int i = 0; i < (KB * KB + NT - 1) / NT; i++)
+                if (a0 + i * (NT / KB) < KB) g[tid + i * NT] = w[b * LD + a0 + i * (NT / KB)];
+        } else {
+#pragma unroll
+            for (int i = 0; i < (KB * KB + NT - 1) / NT; i++)
+                if (a0 + i * (NT / KB) < KB) g[tid + i * NT] = w[(a0 + i * (NT / KB)) * LD + b];
         }
     };
     T *g = gT + (size_t)gb * 3 * TS;
-    put(g, sD, false);
-    put(g + TS, sF, J > M); // J <= M: the shared image of F^T, A(J,J-1) column-major; beyond: row-major
+    put(g, 1, false);
+    put(g + TS, 0, J <= M); // J <= M: A(J,J-1) column-major; beyond: row-major
     if (J < M) {
-        put(g + 2 * TS, sE, false);
-        put(gE + (size_t)gb * TS, sE, true);
+        put(g + 2 * TS, 2, false);
+        put(gE + (size_t)gb * TS, 2, true);
     } else {
-        put(g + 2 * TS, sE, true); // A(J,J+1) column-major
-        if (J > M) put(gE + (size_t)gb * TS, sF, false); // A(J,J-1) column-major
+        put(g + 2 * TS, 2, true); // A(J,J+1) column-major
+        if (J > M) put(gE + (size_t)gb * TS, 0, true); // A(J,J-1) column-major
     }
 }
 
