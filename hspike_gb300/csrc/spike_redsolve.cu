@@ -23,7 +23,7 @@
 //             block: four rows of the products per warp, every operand of both
 //             products requested before the first is used, the vector between
 //             them exchanged through the cluster's shared memory.
-#include "spike_common.cuh"
+#include "spike_slices.cuh"
 
 #include <cooperative_groups.h>
 #include <type_traits>
@@ -715,6 +715,174 @@ __global__ void __launch_bounds__(QNT)
     });
 }
 
+// The same on the tensor cores by exact digit products (spike_slices.cuh), eight
+// columns per CTA: 8 KB^2 FP64 multiply-adds per interface and column are what
+// bounds k_red_resid (102 us at 155 interfaces of 64 rows and 16 columns, 143 at
+// 127 of 128 rows and 8), here 32 and 53.  A CTA forms 64 rows of one equation: its
+// warps take 16 rows and two KB / 32-th parts of the 2 KB columns each, split
+// the tiles' values from registers and the vectors' through shared planes, and
+// add their integer sums there.
+template <int KB> struct RedSl {
+    static constexpr int ROWS = KB < 64 ? KB : 64, KS = KB / 32, WARPS = ROWS / 16 * KS, NT = 32 * WARPS;
+    static constexpr int NC = 8, K = 2 * KB, STEPS = K / 16 / KS, LDX = K + 8; // LDX = 8 mod 64: conflict-free fragments
+    static constexpr int UPW = NC * K / 64 / WARPS;                            // units of 64 values of u per warp
+    static constexpr size_t PL = (size_t)(SL_D + 1) * NC * LDX * 2, PART = (size_t)KS * ROWS * NC * 20;
+    static constexpr size_t SM = ((PL > PART ? PL : PART) + 15) / 16 * 16;
+    static constexpr int CPI = K / ROWS; // CTAs per interface
+};
+template <int KB>
+__global__ void __launch_bounds__(RedSl<KB>::NT)
+    k_red_resid_sl(const float *__restrict__ RP, const float *__restrict__ RQ, const float *__restrict__ RX,
+                   const float *__restrict__ RY, const double *__restrict__ g, const double *__restrict__ u, double *res,
+                   int nif, int nrhs)
+{
+    using Q = RedSl<KB>;
+    constexpr size_t TS = (size_t)KB * KB;
+    __shared__ __align__(16) char pl[Q::SM];
+    __shared__ int er[Q::ROWS], ec[Q::NC];
+    unsigned short *px = (unsigned short *)pl;          // [digit][column][LDX]; plane SL_D: magnitudes
+    long long *xh = (long long *)pl, *xl = xh + Q::KS * Q::ROWS * Q::NC; // partial sums, [ks][column][row]
+    float *xg = (float *)(xl + Q::KS * Q::ROWS * Q::NC);
+    const int i = blockIdx.x / Q::CPI, part = blockIdx.x % Q::CPI, r0 = part * Q::ROWS, half = r0 / KB, q0 = r0 - half * KB;
+    const int h0 = blockIdx.y * Q::NC, nr = min(Q::NC, nrhs - h0);
+    const long long NR = (long long)nif * 2 * KB, b = (long long)i * 2 * KB;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gr = lane >> 2, t = lane & 3;
+    const int wr = warp % (Q::ROWS / 16) * 16, k0 = warp / (Q::ROWS / 16) * Q::STEPS * 16; // this warp's rows and columns
+    const bool far = half ? i + 1 < nif : i > 0; // the neighbouring interface exists
+    const float *A0 = (half ? RQ : RP) + (size_t)i * TS, *A1 = (half ? RY : RX) + (size_t)i * TS;
+    // b-equation: P_i t_{i+1} + X_i b_{i-1}; t-equation: Q_i b_i + Y_i t_{i+2}
+    auto where = [&](int k) {
+        const int kk = k % KB;
+        return k < KB ? b + (half ? 0 : KB) + kk : half ? b + 2 * KB + KB + kk : b - 2 * KB + kk;
+    };
+    float2 av[Q::STEPS][2][2]; // [step][row g, g + 8][columns 2 t, 2 t + 8]
+#pragma unroll
+    for (int s = 0; s < Q::STEPS; s++)
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const int k = k0 + s * 16 + 2 * t + 8 * c;
+                const float *A = (k < KB ? A0 : A1) + (size_t)(q0 + wr + gr + 8 * p) * KB + k % KB;
+                av[s][p][c] = k < KB || far ? *reinterpret_cast<const float2 *>(A) : make_float2(0.f, 0.f);
+            }
+    if (tid < Q::ROWS) er[tid] = 0;
+    if (tid < Q::NC) ec[tid] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+        unsigned m = 0;
+#pragma unroll
+        for (int s = 0; s < Q::STEPS; s++)
+#pragma unroll
+            for (int c = 0; c < 2; c++)
+                m = max(m, max(__float_as_uint(av[s][p][c].x) & 0x7fffffffu, __float_as_uint(av[s][p][c].y) & 0x7fffffffu));
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+        // the FP64 exponent; subnormals at most the smallest normal's, inf and NaN no scale
+        if (t == 0 && m) atomicMax(&er[wr + gr + 8 * p], m >= 0x7f800000u ? 0x7ff : (int)max(m >> 23, 1u) + 1023 - 127);
+    }
+    dep_launch();
+    dep_wait();
+    double v[Q::UPW][2]; // unit x = warp + w WARPS: column x / (K / 64), rows 64 (x % (K / 64)) + 2 lane
+#pragma unroll
+    for (int w = 0; w < Q::UPW; w++) {
+        const int x = warp + w * Q::WARPS, h = x / (Q::K / 64), k = x % (Q::K / 64) * 64 + 2 * lane;
+        const bool live = h < nr && (k < KB || far);
+        v[w][0] = live ? u[(h0 + h) * NR + where(k)] : 0.0;
+        v[w][1] = live ? u[(h0 + h) * NR + where(k + 1)] : 0.0;
+        const unsigned a0 = (unsigned)__double2hiint(v[w][0]) & 0x7fffffffu, l0 = (unsigned)__double2loint(v[w][0]);
+        const unsigned a1 = (unsigned)__double2hiint(v[w][1]) & 0x7fffffffu, l1 = (unsigned)__double2loint(v[w][1]);
+        const unsigned e = __reduce_max_sync(0xffffffffu, max(max(a0, a1) >> 20, (a0 | l0 | a1 | l1) != 0u ? 1u : 0u));
+        if (lane == 0 && e) atomicMax(&ec[h], (int)e);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < Q::UPW; w++) {
+        const int x = warp + w * Q::WARPS, h = x / (Q::K / 64), k = x % (Q::K / 64) * 64 + 2 * lane;
+        const int E = ec[h];
+        const bool live = E >= 64 && E < 0x7ff;
+        unsigned a0, b0, m0, a1, b1, m1;
+        sl_split(live ? v[w][0] : 0.0, live ? E : 64, a0, b0, m0);
+        sl_split(live ? v[w][1] : 0.0, live ? E : 64, a1, b1, m1);
+        unsigned *o = (unsigned *)(px + h * Q::LDX + k);
+        constexpr int ST = Q::NC * Q::LDX / 2;
+        o[0] = sl_digit<0>(a0, b0, a1, b1);
+        o[ST] = sl_digit<1>(a0, b0, a1, b1);
+        o[2 * ST] = sl_digit<2>(a0, b0, a1, b1);
+        o[3 * ST] = sl_digit<3>(a0, b0, a1, b1);
+        o[4 * ST] = sl_digit<4>(a0, b0, a1, b1);
+        o[5 * ST] = sl_digit<5>(a0, b0, a1, b1);
+        o[6 * ST] = sl_digit<6>(a0, b0, a1, b1);
+        o[7 * ST] = sl_digit<7>(a0, b0, a1, b1);
+        o[8 * ST] = m0 | (m1 << 16);
+    }
+    __syncthreads();
+    SlAcc acc;
+    acc.zero();
+    int E[2];
+    bool on[2];
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+        E[p] = er[wr + gr + 8 * p];
+        on[p] = E[p] >= 64 && E[p] < 0x7ff;
+        if (!on[p]) E[p] = 64;
+    }
+#pragma unroll
+    for (int s = 0; s < Q::STEPS; s++) {
+        double w[2][4];
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                w[p][2 * c] = on[p] ? widen(av[s][p][c].x) : 0.0;
+                w[p][2 * c + 1] = on[p] ? widen(av[s][p][c].y) : 0.0;
+            }
+        SlFragA F;
+        F.split(w, E[0], E[1]);
+        const unsigned *xb = (const unsigned *)(px + gr * Q::LDX + k0 + s * 16 + 2 * t);
+        acc.step(F, [&](int d, int q) { return xb[d * (Q::NC * Q::LDX / 2) + 4 * q]; });
+    }
+    __syncthreads(); // the planes have been read
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const int o = (warp / (Q::ROWS / 16) * Q::NC + 2 * t + (e & 1)) * Q::ROWS + wr + gr + 8 * (e >> 1);
+        long long hi, lo;
+        acc.total(e, hi, lo);
+        xh[o] = hi;
+        xl[o] = lo;
+        xg[o] = acc.g[e];
+    }
+    __syncthreads();
+    for (int o = tid; o < Q::ROWS * Q::NC; o += Q::NT) { // (whole warps: one column each)
+        const int h = o / Q::ROWS, rw = o % Q::ROWS;
+        if (h >= nr) break;
+        long long hi = 0, lo = 0;
+        float mg = 0.f;
+#pragma unroll
+        for (int s = 0; s < Q::KS; s++) {
+            hi += xh[s * Q::ROWS * Q::NC + o];
+            lo += xl[s * Q::ROWS * Q::NC + o];
+            mg += xg[s * Q::ROWS * Q::NC + o];
+        }
+        const int Er = er[rw], Ec = ec[h], sc = 56 + Er + Ec - 2 * (1023 + 61);
+        const bool zero = (Er == 0 && Ec < 0x7ff) || (Ec == 0 && Er < 0x7ff);
+        const bool fine = Er >= 64 && Er < 0x7ff && Ec >= 64 && Ec < 0x7ff && mg >= SL_GUARD && sc > -900 && sc < 850;
+        double ax = fine ? sl_round(hi, lo, sc) : 0.0;
+        // the few results outside the scales' reach, one by one in FP64
+        for (unsigned todo = __ballot_sync(0xffffffffu, !fine && !zero); todo; todo &= todo - 1) {
+            const int src = __ffs(todo) - 1, rr = __shfl_sync(0xffffffffu, rw, src);
+            double sum = 0.0;
+            for (int k = lane; k < (far ? 2 * KB : KB); k += 32)
+                sum = fma(widen((k < KB ? A0 : A1)[(size_t)(q0 + rr) * KB + k % KB]), u[(h0 + h) * NR + where(k)], sum);
+            for (int q = 16; q > 0; q >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, q);
+            if (lane == src) ax = sum;
+        }
+        const long long x = (h0 + h) * NR + b + r0 + rw;
+        res[x] = g[x] - u[x] - ax;
+    }
+}
+
 template <class T, int KB, int NRC> int run_red_solve_q(spk_plan *P, int nrhs, int iters, cudaStream_t st)
 {
     using H = typename HighOf<T>::type;
@@ -751,9 +919,18 @@ template <class T, int KB, int NRC> int run_red_solve_q(spk_plan *P, int nrhs, i
         P->launches += 2 * L + 1;
         if (it + 1 < iters) {
             constexpr int RC = NRC > 4 ? 4 : NRC;
-            if (launch_dep(k_red_resid<T, KB, RC>, dim3(P->n_iface * Q::CS, (nrhs + RC - 1) / RC), QNT, 0, 1, true, st,
+            int rc = SPK_OK;
+            // (one column: the FP64 pipe is done sooner, 18 against 32 us at 255 interfaces of 64
+            // rows; two columns 30 against 25 us at 127 of 128 rows)
+            if constexpr (std::is_same<T, float>::value && NRC > 1) {
+                using S = RedSl<KB>;
+                rc = launch_dep(k_red_resid_sl<KB>, dim3(P->n_iface * S::CPI, (nrhs + S::NC - 1) / S::NC), S::NT, 0, 1,
+                                true, st, (const T *)P->d_crP, (const T *)P->d_crQ, cX, cY, (const H *)P->d_g,
+                                (const H *)P->d_u, (H *)P->d_rr, P->n_iface, nrhs);
+            } else if (launch_dep(k_red_resid<T, KB, RC>, dim3(P->n_iface * Q::CS, (nrhs + RC - 1) / RC), QNT, 0, 1, true, st,
                            (const T *)P->d_crP, (const T *)P->d_crQ, cX, cY, (const H *)P->d_g, (const H *)P->d_u, (H *)P->d_rr, P->n_iface, nrhs) != SPK_OK)
-                return SPK_ECUDA;
+                rc = SPK_ECUDA;
+            if (rc != SPK_OK) return rc;
             P->launches++;
         }
     }
