@@ -165,179 +165,267 @@ __global__ void __launch_bounds__(NTOf<KB>::value)
     }
 }
 
-// ---------------------------------------------------------------- tensor-core products
-// The reduced system's 2KB x 2KB block products for KB >= 64 (FP32 factors)
-// run on the tensor cores: warp-level mma.sync m16n8k8 with TF32 operands,
-// each FP32 operand split into a TF32 high part and a TF32 remainder, and
-// the three significant partial products (lo*hi, hi*lo, hi*hi) accumulated
-// in FP32, which keeps FP32 accuracy.  Warp w of the CTA (KB*KB/512 warps:
-// the Tile kernels' own thread count) owns the 32 x 16 output block at rows
-// 32 (w / (KB/16)), columns 16 (w % (KB/16)); operands are shared tiles in
-// the Tile layout (row-major, row stride KB + 4).
-__device__ __forceinline__ void tf32_split(float x, uint32_t &hi, uint32_t &lo)
-{
-    uint32_t h, l;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(x));
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(x - __uint_as_float(h)));
-    hi = h;
-    lo = l;
-}
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2])
-{
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-                 "{%0,%1,%2,%3};\n"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-using TcAcc = float[2][2][4];
-__device__ __forceinline__ void tc_zero(TcAcc &acc)
-{
+// ---------------------------------------------------------------- FP32, KB >= 32: products by column slices
+// A level has few blocks (63, 32, 16, ... of 127 interfaces), so its time is that
+// of one block.  Columns of a product's right operand are independent through
+// all of k_cr_odd's and k_cr_even's formulas but the inverse, so every block's
+// products are split into slices of CW columns: a CTA streams the left operands
+// through a ring of 32-column pieces while its slice of the right one stays in
+// shared memory (FP32 multiply-adds: 128 a clock and SM, where three TF32
+// products come to 85).  Level by level: S and its inverse (one CTA; from 128 rows
+// on S has a launch of its own), the other quadrants, the even blocks, each launched
+// while the one before runs out.  A block to a CTA, with TF32 products: 1,090 us
+// for 127 interfaces of 128 rows (99 for an odd block, 35 for an even one), 607
+// so; 299 for 155 of 64 rows, 230; 195 for 303 of 32 rows, 136.
+template <int KB, int CW> struct ColMul {
+    static constexpr int NT = 256, NS = KB / CW, KC = 32, ST = 4;
+    static constexpr int TX = CW / 4, RS = NT / TX, RPT = KB / RS; // a thread's rows, RS apart, of 4 columns
+    static constexpr int LDA = KC + 4, LDB = CW + 4, NC = KB / KC; // conflict-free 16-byte reads
+    static constexpr int RING = ST * KB * LDA, SLICE = KB * LDB;
+    static constexpr size_t SMEM = sizeof(float) * (RING + 2 * SLICE);
+    using Acc = float[RPT][4];
+    float *ring, *b0, *b1; // pieces of the left operands; two slices
+    const float *A[2];     // the left operands of the first NC pieces and of the others
+    int total;
+    __device__ __forceinline__ ColMul(char *sm, int passes) : ring((float *)sm), b0(ring + RING), b1(b0 + SLICE), total(passes * NC) {}
+    static __device__ __forceinline__ int row(int i) { return threadIdx.x / TX + RS * i; }
+    static __device__ __forceinline__ int col() { return threadIdx.x % TX * 4; }
+    __device__ __forceinline__ void issue(int c) const
+    {
+        if (c < total) {
+            const float *src = A[c / NC] + c % NC * KC;
+            float *dst = ring + c % ST * KB * LDA;
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+            for (int q = threadIdx.x; q < KB * KC / 4; q += NT)
+                cp_async16(dst + q / (KC / 4) * LDA + q % (KC / 4) * 4, src + (size_t)(q / (KC / 4)) * KB + q % (KC / 4) * 4);
+        }
+        cp_async_commit(); // (empty past the end: the waits count groups)
+    }
+    // columns [c0, c0 + CW) of a global tile, with the first piece's group
+    static __device__ __forceinline__ void slice(float *s, const float *g, int c0)
+    {
 #pragma unroll
-        for (int j = 0; j < 2; j++)
+        for (int q = threadIdx.x; q < KB * CW / 4; q += NT)
+            cp_async16(s + q / (CW / 4) * LDB + q % (CW / 4) * 4, g + (size_t)(q / (CW / 4)) * KB + c0 + q % (CW / 4) * 4);
+    }
+    __device__ __forceinline__ void start() const
+    {
+        for (int c = 0; c < ST - 1; c++) issue(c);
+    }
+    // acc = A[p] b (and acc2 = A[p] b2): pieces p NC .. p NC + NC - 1
+    template <bool TWO> __device__ __forceinline__ void pass(int p, Acc &acc, const float *b, Acc &acc2, const float *b2) const
+    {
 #pragma unroll
-            for (int e = 0; e < 4; e++) acc[i][j][e] = 0.f;
-}
-// acc += A B (A, B: KB x KB shared tiles, row-major, row stride KB + 4)
-template <int KB> __device__ __forceinline__ void tc_mm(TcAcc &acc, const float *A, const float *B)
-{
-    constexpr int LD = TileLD<float, KB>::value;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int r0 = (warp / (KB / 16)) * 32, c0 = (warp % (KB / 16)) * 16;
+        for (int i = 0; i < RPT; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[i][j] = acc2[i][j] = 0.f;
+        const int cc = col(), r0 = row(0);
+        for (int c = p * NC; c < (p + 1) * NC; c++) {
+            cp_async_wait_n<ST - 2>();
+            __syncthreads(); // the piece is everyone's, and the one before it has been used
+            issue(c + ST - 1);
+            const float *a0 = ring + c % ST * KB * LDA + r0 * LDA, *bb = b + c % NC * KC * LDB + cc, *bb2 = b2 + c % NC * KC * LDB + cc;
 #pragma unroll 2
-    for (int k0 = 0; k0 < KB; k0 += 8) {
-        uint32_t ah[2][4], al[2][4], bh[2][2], bl[2][2];
+            for (int k = 0; k < KC; k += 4) {
+                float a[RPT][4];
 #pragma unroll
-        for (int i = 0; i < 2; i++) { // A fragment: (g, t), (g + 8, t), (g, t + 4), (g + 8, t + 4)
-            const float *Ar = A + (r0 + i * 16 + g) * LD + k0 + t;
-            tf32_split(Ar[0], ah[i][0], al[i][0]);
-            tf32_split(Ar[8 * LD], ah[i][1], al[i][1]);
-            tf32_split(Ar[4], ah[i][2], al[i][2]);
-            tf32_split(Ar[8 * LD + 4], ah[i][3], al[i][3]);
-        }
+                for (int i = 0; i < RPT; i++) vld<float, 4>(a[i], a0 + RS * i * LDA + k);
 #pragma unroll
-        for (int j = 0; j < 2; j++) { // B fragment: (t, g), (t + 4, g)
-            const float *Bc = B + (k0 + t) * LD + c0 + j * 8 + g;
-            tf32_split(Bc[0], bh[j][0], bl[j][0]);
-            tf32_split(Bc[4 * LD], bh[j][1], bl[j][1]);
-        }
+                for (int q = 0; q < 4; q++) {
+                    float x[4];
+                    vld<float, 4>(x, bb + (k + q) * LDB);
 #pragma unroll
-        for (int i = 0; i < 2; i++)
+                    for (int i = 0; i < RPT; i++)
 #pragma unroll
-            for (int j = 0; j < 2; j++) {
-                mma_tf32(acc[i][j], al[i], bh[j]);
-                mma_tf32(acc[i][j], ah[i], bl[j]);
-                mma_tf32(acc[i][j], ah[i], bh[j]);
+                        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i][q], x[j], acc[i][j]);
+                    if constexpr (TWO) {
+                        vld<float, 4>(x, bb2 + (k + q) * LDB);
+#pragma unroll
+                        for (int i = 0; i < RPT; i++)
+#pragma unroll
+                            for (int j = 0; j < 4; j++) acc2[i][j] = fmaf(a[i][q], x[j], acc2[i][j]);
+                    }
+                }
             }
+        }
+    }
+    // f(row, first of four columns of the slice, i) per row of this thread
+    template <class F> static __device__ __forceinline__ void each(F f)
+    {
+#pragma unroll
+        for (int i = 0; i < RPT; i++) f(row(i), col(), i);
+    }
+};
+
+// columns [c0, c0 + CW) of S = I - Q P of odd block j, where M11 goes
+template <int KB, int CW>
+__global__ void __launch_bounds__(256)
+    k_cr_schur(const float *__restrict__ Pl, const float *__restrict__ Ql, int first, int stride, float *M)
+{
+    using C = ColMul<KB, CW>;
+    constexpr size_t TS = (size_t)KB * KB;
+    const int c0 = blockIdx.y * CW;
+    const size_t o = (size_t)(first + blockIdx.x * stride) * TS;
+    float *S = M + (size_t)blockIdx.x * 4 * TS + 3 * TS;
+    extern __shared__ __align__(16) char sm[];
+    C m(sm, 1);
+    m.A[0] = Ql + o;
+    dep_launch();
+    dep_wait();
+    C::slice(m.b0, Pl + o, c0);
+    m.start();
+    typename C::Acc a, u;
+    m.template pass<false>(0, a, m.b0, u, m.b0);
+    C::each([&](int r, int c, int i) {
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = (r == c0 + c + j ? 1.f : 0.f) - a[i][j];
+        vst<float, 4>(S + (size_t)r * KB + c0 + c, v);
+    });
+}
+// M11 = S^{-1} in place
+template <int KB>
+__global__ void __launch_bounds__(256) k_cr_inv(float *M, unsigned *err)
+{
+    constexpr int LD = KB + 4;
+    float *S = M + ((size_t)blockIdx.x * 4 + 3) * KB * KB;
+    extern __shared__ __align__(16) char sm[];
+    float *s = (float *)sm;
+    dep_launch();
+    dep_wait();
+    for (int q = threadIdx.x; q < KB * KB / 4; q += 256) {
+        float v[4];
+        vld<float, 4>(v, S + q * 4);
+        vst<float, 4>(s + q / (KB / 4) * LD + q % (KB / 4) * 4, v);
+    }
+    __syncthreads();
+    const bool ok = BlkInv<256, LD>::template run<KB>(s);
+    if (!ok) atomicOr(err, SPK_DEV_ERR_PIVOT);
+    for (int q = threadIdx.x; q < KB * KB / 4; q += 256) {
+        float v[4];
+        vld<float, 4>(v, s + q / (KB / 4) * LD + q % (KB / 4) * 4);
+        vst<float, 4>(S + q * 4, v);
     }
 }
-// f(row, col, value) for every accumulator element this thread holds:
-// (g, 2t), (g, 2t + 1), (g + 8, 2t), (g + 8, 2t + 1) of each 16 x 8 block
-template <int KB, class F> __device__ __forceinline__ void tc_each(const TcAcc &acc, F f)
-{
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int r0 = (warp / (KB / 16)) * 32, c0 = (warp % (KB / 16)) * 16;
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 2; j++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) f(r0 + i * 16 + g + (e >> 1) * 8, c0 + j * 8 + 2 * t + (e & 1), acc[i][j][e]);
-}
-
-// k_cr_odd with tensor-core products: S = I - Q P, M11 = S^{-1} (the Tile
-// inverse), M10 = -M11 Q, M01 = -P M11, M00 = I - P M10.
+// both at once for tiles whose S one CTA forms soon enough
 template <int KB>
-__global__ void __launch_bounds__(NTOf<KB>::value)
-    k_cr_odd_tc(const float *__restrict__ Pl, const float *__restrict__ Ql, int first, int stride, float *M,
-                unsigned *err)
+__global__ void __launch_bounds__(256)
+    k_cr_schur_inv(const float *__restrict__ Pl, const float *__restrict__ Ql, int first, int stride, float *M,
+                   unsigned *err)
 {
-    constexpr int NT = NTOf<KB>::value, LD = TileLD<float, KB>::value;
-    using TL = Tile<float, KB, NT>;
-    constexpr size_t TS = (size_t)KB * KB;
-    static_assert(NT == KB * KB / 16, "one warp per 32 x 16 output block");
-    const int j = first + blockIdx.x * stride;
-    float *Mj = M + (size_t)blockIdx.x * 4 * TS;
-    extern __shared__ char smraw[];
-    float *sP = (float *)smem_align(smraw), *sQ = sP + TL::ELEMS, *sH = sQ + TL::ELEMS;
-    float *buf = sH + TL::ELEMS;
-    TL t(threadIdx.x);
-    typename TL::Reg a;
-    TcAcc acc;
-    ld<float, KB>(sP, Pl + (size_t)j * TS);
-    ld<float, KB>(sQ, Ql + (size_t)j * TS);
+    constexpr int LD = KB + 4;
+    using B = BlkMul<KB, 256, LD>;
+    const size_t o = (size_t)(first + blockIdx.x * stride) * KB * KB;
+    float *S = M + ((size_t)blockIdx.x * 4 + 3) * KB * KB;
+    extern __shared__ __align__(16) char sm[];
+    float *p = (float *)sm, *q = p + KB * LD;
+    dep_launch();
+    dep_wait();
+    for (int i = threadIdx.x; i < KB * KB / 4; i += 256) {
+        cp_async16(p + i / (KB / 4) * LD + i % (KB / 4) * 4, Pl + o + i * 4);
+        cp_async16(q + i / (KB / 4) * LD + i % (KB / 4) * 4, Ql + o + i * 4);
+    }
+    cp_async_commit();
+    cp_async_wait_all();
     __syncthreads();
-    tc_zero(acc);
-    tc_mm<KB>(acc, sQ, sP);
-    tc_each<KB>(acc, [&](int r, int c, float v) { sH[r * LD + c] = (r == c ? 1.f : 0.f) - v; }); // S
+    typename B::Acc a;
+    B::mul(threadIdx.x, a, q, p);
     __syncthreads();
-    t.rload(a, sH);
+    B::template put<false, true>(threadIdx.x, p, a);
     __syncthreads();
-    bool ok;
-    if constexpr (KB == 64)
-        ok = t.inverse_blk(a, sH);
-    else
-        ok = t.inverse(a, buf);
-    if (!ok && threadIdx.x == 0) atomicOr(err, SPK_DEV_ERR_PIVOT);
+    if (threadIdx.x < KB) p[threadIdx.x * LD + threadIdx.x] += 1.f;
     __syncthreads();
-    t.rstore(sH, a); // M11
-    t.gstore(Mj + 3 * TS, a);
-    __syncthreads();
-    tc_zero(acc);
-    tc_mm<KB>(acc, sH, sQ);
-    tc_each<KB>(acc, [&](int r, int c, float v) { Mj[2 * TS + r * KB + c] = -v; }); // M10
-    __syncthreads(); // every read of Q is done
-    tc_each<KB>(acc, [&](int r, int c, float v) { sQ[r * LD + c] = -v; });
-    tc_zero(acc);
-    tc_mm<KB>(acc, sP, sH);
-    tc_each<KB>(acc, [&](int r, int c, float v) { Mj[TS + r * KB + c] = -v; }); // M01
-    __syncthreads();
-    tc_zero(acc);
-    tc_mm<KB>(acc, sP, sQ);
-    tc_each<KB>(acc, [&](int r, int c, float v) { Mj[r * KB + c] = (r == c ? 1.f : 0.f) - v; }); // M00
+    const bool ok = BlkInv<256, LD>::template run<KB>(p);
+    if (!ok) atomicOr(err, SPK_DEV_ERR_PIVOT);
+    for (int i = threadIdx.x; i < KB * KB / 4; i += 256) {
+        float v[4];
+        vld<float, 4>(v, p + i / (KB / 4) * LD + i % (KB / 4) * 4);
+        vst<float, 4>(S + i * 4, v);
+    }
 }
-
-// k_cr_even with tensor-core products: blockIdx.y picks the result
+// columns [c0, c0 + CW) of M10 = -M11 Q, M01 = -P M11, M00 = I - P M10
+template <int KB, int CW>
+__global__ void __launch_bounds__(256)
+    k_cr_quads(const float *__restrict__ Pl, const float *__restrict__ Ql, int first, int stride, float *M)
+{
+    using C = ColMul<KB, CW>;
+    constexpr size_t TS = (size_t)KB * KB;
+    const int c0 = blockIdx.y * CW;
+    const size_t o = (size_t)(first + blockIdx.x * stride) * TS;
+    float *Mj = M + (size_t)blockIdx.x * 4 * TS;
+    extern __shared__ __align__(16) char sm[];
+    C m(sm, 2);
+    m.A[0] = Mj + 3 * TS;
+    m.A[1] = Pl + o;
+    dep_launch();
+    dep_wait();
+    C::slice(m.b0, Ql + o, c0);
+    C::slice(m.b1, Mj + 3 * TS, c0);
+    m.start();
+    typename C::Acc a, u;
+    m.template pass<false>(0, a, m.b0, u, m.b0);
+    __syncthreads(); // Q's slice has been used
+    C::each([&](int r, int c, int i) {
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = -a[i][j];
+        vst<float, 4>(m.b0 + r * C::LDB + c, v);
+        vst<float, 4>(Mj + 2 * TS + (size_t)r * KB + c0 + c, v);
+    });
+    m.template pass<true>(1, a, m.b1, u, m.b0); // (a barrier before its first read)
+    C::each([&](int r, int c, int i) {
+        float v[4], w[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            v[j] = -a[i][j];
+            w[j] = (r == c0 + c + j ? 1.f : 0.f) - u[i][j];
+        }
+        vst<float, 4>(Mj + TS + (size_t)r * KB + c0 + c, v);
+        vst<float, 4>(Mj + (size_t)r * KB + c0 + c, w);
+    });
+}
+// columns [c0, c0 + CW) of an even block's result blockIdx.y % 4 (k_cr_even)
 //   0: P' = P_i - X_i (M01 Y)_{i-1}   1: Q' = Q_i - Y_i (M10 X)_{i+1}
 //   2: X' = -X_i (M00 X)_{i-1}        3: Y' = -Y_i (M11 Y)_{i+1}
-template <int KB>
-__global__ void __launch_bounds__(NTOf<KB>::value)
-    k_cr_even_tc(const float *__restrict__ Pl, const float *__restrict__ Ql, const float *__restrict__ Xl,
-                 const float *__restrict__ Yl, const float *__restrict__ Ml, int cnt, float *Pn, float *Qn,
-                 float *Xn, float *Yn)
+template <int KB, int CW>
+__global__ void __launch_bounds__(256)
+    k_cr_even_cols(const float *__restrict__ Pl, const float *__restrict__ Ql, const float *__restrict__ Xl,
+                   const float *__restrict__ Yl, const float *__restrict__ Ml, int cnt, float *Pn, float *Qn, float *Xn,
+                   float *Yn)
 {
-    constexpr int NT = NTOf<KB>::value, LD = TileLD<float, KB>::value;
-    using TL = Tile<float, KB, NT>;
+    using C = ColMul<KB, CW>;
     constexpr size_t TS = (size_t)KB * KB;
-    const int i = 2 * blockIdx.x, a_out = blockIdx.x, which = blockIdx.y;
-    const bool left = i - 1 >= 0, right = i + 1 < cnt;
-    const bool has = (which == 0 || which == 2) ? left : right;
-    const float *base = which == 0 ? Pl + (size_t)i * TS : which == 1 ? Ql + (size_t)i * TS : nullptr;
-    float *out = (which == 0 ? Pn : which == 1 ? Qn : which == 2 ? Xn : Yn) + (size_t)a_out * TS;
-    if (!has) { // no neighbour on this side: P' = P_i, Q' = Q_i, X' = Y' = 0
-        for (int q = threadIdx.x; q < KB * KB; q += NT) out[q] = base ? base[q] : 0.f;
-        return;
+    const int i = 2 * blockIdx.x, w = blockIdx.y % 4, c0 = blockIdx.y / 4 * CW;
+    const bool lft = w == 0 || w == 2, has = lft ? i > 0 : i + 1 < cnt;
+    const int j = lft ? i - 1 : i + 1;
+    const float *base = w == 0 ? Pl + (size_t)i * TS : w == 1 ? Ql + (size_t)i * TS : nullptr;
+    float *out = (w == 0 ? Pn : w == 1 ? Qn : w == 2 ? Xn : Yn) + (size_t)blockIdx.x * TS;
+    extern __shared__ __align__(16) char sm[];
+    C m(sm, 2);
+    dep_launch();
+    dep_wait();
+    typename C::Acc a, u;
+    if (has) {
+        m.A[0] = Ml + ((size_t)(j / 2) * 4 + (w == 0 ? 1 : w == 1 ? 2 : w == 2 ? 0 : 3)) * TS;
+        m.A[1] = (lft ? Xl : Yl) + (size_t)i * TS;
+        C::slice(m.b0, (w == 0 || w == 3 ? Yl : Xl) + (size_t)j * TS, c0);
+        m.start();
+        m.template pass<false>(0, a, m.b0, u, m.b0);
+        C::each([&](int r, int c, int q) { vst<float, 4>(m.b1 + r * C::LDB + c, a[q]); });
+        m.template pass<false>(1, a, m.b1, u, m.b1); // (a barrier before its first read)
+    } else { // no neighbour on this side: P' = P_i, Q' = Q_i, X' = Y' = 0
+#pragma unroll
+        for (int q = 0; q < C::RPT; q++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) a[q][k] = 0.f;
     }
-    const float *Mnb = Ml + (size_t)(left && (which == 0 || which == 2) ? (i - 2) / 2 : i / 2) * 4 * TS;
-    const float *Lt = (which == 0 || which == 2 ? Xl : Yl) + (size_t)i * TS;
-    const float *Mq = Mnb + (size_t)(which == 0 ? 1 : which == 1 ? 2 : which == 2 ? 0 : 3) * TS;
-    const float *Rt = (which == 0 || which == 3 ? Yl : Xl) + (size_t)(which == 0 || which == 2 ? i - 1 : i + 1) * TS;
-    extern __shared__ char smraw[];
-    float *sA = (float *)smem_align(smraw), *sB = sA + TL::ELEMS, *sC = sB + TL::ELEMS;
-    ld<float, KB>(sA, Mq);
-    ld<float, KB>(sB, Rt);
-    __syncthreads();
-    TcAcc acc;
-    tc_zero(acc);
-    tc_mm<KB>(acc, sA, sB);
-    tc_each<KB>(acc, [&](int r, int c, float v) { sC[r * LD + c] = v; });
-    __syncthreads();
-    ld<float, KB>(sA, Lt);
-    __syncthreads();
-    tc_zero(acc);
-    tc_mm<KB>(acc, sA, sC);
-    tc_each<KB>(acc, [&](int r, int c, float v) { out[r * KB + c] = (base ? base[r * KB + c] : 0.f) - v; });
+    C::each([&](int r, int c, int q) {
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (base) vld<float, 4>(v, base + (size_t)r * KB + c0 + c);
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] -= a[q][k];
+        vst<float, 4>(out + (size_t)r * KB + c0 + c, v);
+    });
 }
 
 // ------------------------------------------------------------ KB <= 16: segments of several levels
@@ -537,6 +625,71 @@ template <class T, int KB> int run_red_factor_s(spk_plan *P, cudaStream_t st)
     return run(k_rf_seg<T, KB, NTT>, 1, NTT, bytes(lv.cnt[lt], lv.L - lt, true), lt, lv.L, 1);
 }
 
+template <int KB> int run_red_factor_c(spk_plan *P, cudaStream_t st)
+{
+    using C = ColMul<KB, 32>;
+    constexpr int FINE = KB == 32 ? 32 : 16;
+    using C2 = ColMul<KB, FINE>;
+    constexpr size_t TS = (size_t)KB * KB, INV = sizeof(float) * KB * (KB + 4);
+    static bool attr = false;
+    if (!attr) {
+        const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        if (cudaFuncSetAttribute(k_cr_schur<KB, 32>, a, (int)C::SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_cr_quads<KB, 32>, a, (int)C::SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_cr_even_cols<KB, 32>, a, (int)C::SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_cr_schur<KB, FINE>, a, (int)C2::SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_cr_quads<KB, FINE>, a, (int)C2::SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_cr_even_cols<KB, FINE>, a, (int)C2::SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_cr_schur_inv<KB>, a, (int)(2 * INV)) != cudaSuccess ||
+            cudaFuncSetAttribute(k_cr_inv<KB>, a, (int)INV) != cudaSuccess)
+            return SPK_ECUDA;
+        attr = true;
+    }
+    float *cP = (float *)P->d_crP, *cQ = (float *)P->d_crQ, *cX = (float *)P->d_crX, *cY = (float *)P->d_crY,
+          *cM = (float *)P->d_crM;
+    bool dep = false; // (what ran before these kernels does not let them start early)
+    int rc = SPK_OK;
+    auto run = [&](auto kern, dim3 grid, size_t smem, auto... args) {
+        if (rc == SPK_OK) rc = launch_dep(kern, grid, C::NT, smem, 1, dep, st, args...);
+        dep = true;
+        P->launches++;
+    };
+    auto odd = [&](const float *p, const float *q, int first, int stride, int count, float *M) {
+        // slices of 16 columns while they leave an SM to each
+        const bool fine = count * C2::NS <= 152;
+        if constexpr (KB <= 64) {
+            run(k_cr_schur_inv<KB>, dim3(count), 2 * INV, p, q, first, stride, M, P->d_err);
+        } else {
+            if (fine)
+                run(k_cr_schur<KB, FINE>, dim3(count, C2::NS), C2::SMEM, p, q, first, stride, M);
+            else
+                run(k_cr_schur<KB, 32>, dim3(count, C::NS), C::SMEM, p, q, first, stride, M);
+            run(k_cr_inv<KB>, dim3(count), INV, M, P->d_err);
+        }
+        if (fine)
+            run(k_cr_quads<KB, FINE>, dim3(count, C2::NS), C2::SMEM, p, q, first, stride, M);
+        else
+            run(k_cr_quads<KB, 32>, dim3(count, C::NS), C::SMEM, p, q, first, stride, M);
+    };
+    for (int l = 0; l < P->cr_levels; l++) {
+        const int cnt = P->cr_count[l];
+        const size_t o = (size_t)P->cr_off[l] * TS, on = (size_t)P->cr_off[l + 1] * TS;
+        float *Ml = cM + (size_t)P->cr_moff[l] * 4 * TS;
+        if (cnt / 2 > 0) odd(cP + o, cQ + o, 1, 2, cnt / 2, Ml);
+        auto even = [&](auto kern, int ns, size_t smem) {
+            run(kern, dim3((cnt + 1) / 2, 4 * ns), smem, (const float *)cP + o, (const float *)cQ + o,
+                (const float *)cX + o, (const float *)cY + o, (const float *)Ml, cnt, cP + on, cQ + on, cX + on, cY + on);
+        };
+        if ((cnt + 1) / 2 * 4 * C2::NS <= 152)
+            even(k_cr_even_cols<KB, FINE>, C2::NS, C2::SMEM);
+        else
+            even(k_cr_even_cols<KB, 32>, C::NS, C::SMEM);
+    }
+    const size_t o = (size_t)P->cr_off[P->cr_levels] * TS; // the top block
+    odd(cP + o, cQ + o, 0, 1, 1, cM + (size_t)P->cr_moff[P->cr_levels] * 4 * TS);
+    return rc;
+}
+
 template <class T, int KB> int run_red_factor(spk_plan *P, cudaStream_t st)
 {
     using S = RedSmem<T, KB>;
@@ -554,24 +707,17 @@ template <class T, int KB> int run_red_factor(spk_plan *P, cudaStream_t st)
     }
     if constexpr (KB <= 16) {
         return run_red_factor_s<T, KB>(P, st);
+    } else if constexpr (std::is_same<T, float>::value) {
+        return run_red_factor_c<KB>(P, st);
     } else {
-    // FP32 factors with 64- or 128-row tiles: the block products on the tensor cores
-    constexpr bool TC = std::is_same<T, float>::value && (KB == 64 || KB == 128);
-    // FP64 with 64-row tiles: likewise, by exact digit products (spike_emu64.cu)
+    // FP64 with 64-row tiles: the products on the tensor cores, by exact digits (spike_emu64.cu)
     constexpr bool EMU = std::is_same<T, double>::value && KB == 64;
     static bool attr = false;
     if (!attr) {
-        if constexpr (!TC && !EMU) {
+        if constexpr (!EMU) {
             if (cudaFuncSetAttribute(k_cr_odd<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes) !=
                     cudaSuccess ||
                 cudaFuncSetAttribute(k_cr_even<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes) !=
-                    cudaSuccess)
-                return SPK_ECUDA;
-        }
-        if constexpr (TC) {
-            if (cudaFuncSetAttribute(k_cr_odd_tc<KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes) !=
-                    cudaSuccess ||
-                cudaFuncSetAttribute(k_cr_even_tc<KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes) !=
                     cudaSuccess)
                 return SPK_ECUDA;
         }
@@ -580,8 +726,6 @@ template <class T, int KB> int run_red_factor(spk_plan *P, cudaStream_t st)
     auto odd = [&](const T *Pp, const T *Qp, int first, int stride, int count, T *Mo) {
         if constexpr (EMU)
             spk_emu_cr_odd(Pp, Qp, first, stride, count, Mo, P->d_err, st);
-        else if constexpr (TC)
-            k_cr_odd_tc<KB><<<count, NT, S::bytes, st>>>(Pp, Qp, first, stride, Mo, P->d_err);
         else
             k_cr_odd<T, KB><<<count, NT, S::bytes, st>>>(Pp, Qp, first, stride, Mo, P->d_err);
     };
@@ -597,9 +741,6 @@ template <class T, int KB> int run_red_factor(spk_plan *P, cudaStream_t st)
         }
         if constexpr (EMU)
             spk_emu_cr_even(cP + o, cQ + o, cX + o, cY + o, Ml, cnt, cP + on, cQ + on, cX + on, cY + on, st);
-        else if constexpr (TC)
-            k_cr_even_tc<KB><<<dim3(neven, 4), NT, S::bytes, st>>>(cP + o, cQ + o, cX + o, cY + o, Ml, cnt, cP + on,
-                                                                   cQ + on, cX + on, cY + on);
         else
             k_cr_even<T, KB><<<dim3(neven, 4), NT, S::bytes, st>>>(cP + o, cQ + o, cX + o, cY + o, Ml, cnt, cP + on,
                                                                    cQ + on, cX + on, cY + on);
