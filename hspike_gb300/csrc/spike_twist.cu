@@ -25,6 +25,7 @@
 //               W's C^ top-down through L, V's B^ bottom-up through U
 //   k_tw_merge  (grid p)     block M: L_M, G_M and X_M of both spikes
 //   k_tw_bwd    (grid p x 4) back substitution of W and V, top and bottom halves
+//               (k_tw_bwd_vw for FP32 64-row tiles: both spikes of a half together)
 //   k_tw_lu_w / k_tw_sweep_w / k_tw_bwd_w   the elimination chains, forward
 //               sweeps and back substitution
 //               for FP32 16- and 32-row tiles on one warp per chain (TileW), four
@@ -785,6 +786,164 @@ __global__ void __launch_bounds__(TwCfg<T, KB>::NT_PROD, 4)
     bE.drain();
 }
 
+// k_tw_bwd for FP32 64-row tiles: V and W of one half together, 32 columns of each
+// per CTA.  Both spikes meet the same G and E tiles, so their columns are one right
+// operand, of which 64 threads take 8 x 8 sub-tiles (rows 4 ty .. and 32 + 4 ty ..,
+// columns 4 tx .. of either spike).  Shared memory hands a warp 128 bytes a clock
+// whatever its lanes share: with 8 x 4 sub-tiles that was 12 clocks of reads for 8
+// of multiply-adds (L1 at 84 %, FMA pipe at 44 %), here it is 16 for 16.  The tiles
+// come in quarters of 16 columns through two buffers and E's zero quarters are
+// left out, evenly for both warps; eight CTAs fit an SM, so that the four of each
+// partition spread over the SMs without a second round.  The two CTAs of a half are a cluster: X_J (column-major) overwrites Z_J
+// (row-major), which both must have read by then.  n = 2,000,000, k = 64:
+// 1,645 -> 1,565 us at 256 partitions (6.7 CTAs an SM, whose fullest quarter sets the
+// time), 1,597 -> 1,363 at 304.
+struct TwVW {
+    static constexpr int KB = 64, NT = 64, NC = 32, LDX = 2 * NC + 4, PK = 16, PIECE = PK * KB;
+    static constexpr size_t SMEM = 64 + sizeof(float) * (KB * LDX + 2 * PIECE);
+};
+__device__ __forceinline__ void ld4(float *d, const float *p)
+{
+    const float4 v = *reinterpret_cast<const float4 *>(p);
+    d[0] = v.x, d[1] = v.y, d[2] = v.z, d[3] = v.w;
+}
+__device__ __forceinline__ void st4(float *p, const float *v)
+{
+    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__global__ void __launch_bounds__(TwVW::NT, 8)
+    k_tw_bwd_vw(const int *__restrict__ blk_off, int p, const float *__restrict__ gG, const float *__restrict__ gE,
+                float *gV, float *gW, int part0, unsigned *err)
+{
+    constexpr int KB = TwVW::KB, LDX = TwVW::LDX, PK = TwVW::PK, PIECE = TwVW::PIECE, NC = TwVW::NC;
+    constexpr size_t TS = (size_t)KB * KB;
+    const int part = blockIdx.x / 2 + part0, cb = blockIdx.x % 2 * NC;
+    const bool top = blockIdx.y == 0, doV = part < p - 1, doW = part > 0;
+    const int N = blk_off[part + 1] - blk_off[part], M = N / 2;
+    const size_t tb = (size_t)blk_off[part] * TS;
+    const int cnt = top ? M : N - 1 - M; // steps
+    float *gZ = top ? (doW ? gW : nullptr) : doV ? gV : nullptr; // the spike with a forward sweep
+    extern __shared__ __align__(16) char smraw[];
+    uint64_t *bars = (uint64_t *)smraw;
+    float *sX = (float *)(smraw + 64), *ring = sX + KB * LDX;
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3, w = threadIdx.x >> 5;
+    auto row = [&](int i) { return 4 * ty + (i & 3) + 32 * (i >> 2); };
+    if (threadIdx.x == 0) {
+        mbar_init(bars, 1);
+        mbar_init(bars + 1, 1);
+        mbar_init_fence();
+    }
+    __syncthreads();
+    auto block = [&](int i) { return top ? M - 1 - i : M + 1 + i; };
+    // piece s: step s / 8; E's four quarters, then G's
+    auto issue = [&](int s) {
+        if (threadIdx.x == 0 && s < 8 * cnt) {
+            fence_proxy_async();
+            mbar_arrive_expect_tx(bars + (s & 1), PIECE * 4);
+            bulk_g2s(ring + (s & 1) * PIECE, (s & 4 ? gG : gE) + tb + (size_t)block(s >> 3) * TS + (s & 3) * PIECE,
+                     PIECE * 4, bars + (s & 1));
+        }
+    };
+    issue(0);
+    issue(1);
+    for (int q = threadIdx.x; q < KB * NC; q += TwVW::NT) { // X_M, from column-major
+        const int c = q / KB, r = q % KB;
+        sX[r * LDX + c] = doV ? gV[tb + (size_t)M * TS + cb * KB + q] : 0.f;
+        sX[r * LDX + NC + c] = doW ? gW[tb + (size_t)M * TS + cb * KB + q] : 0.f;
+    }
+    float acc[8][8]; // columns 4 tx + j of V, then of W
+    auto start = [&](int i) { // Z of step i where the spike has one
+#pragma unroll
+        for (int a = 0; a < 8; a++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc[a][j] = 0.f;
+        if (gZ && i < cnt) {
+            const float *z = gZ + tb + (size_t)block(i) * TS + cb + 4 * tx;
+            if (top) {
+#pragma unroll
+                for (int a = 0; a < 8; a++) ld4(acc[a] + 4, z + row(a) * KB);
+            } else {
+#pragma unroll
+                for (int a = 0; a < 8; a++) ld4(acc[a], z + row(a) * KB);
+            }
+        }
+    };
+    // acc (+|-)= the piece's columns times rows kb .. of X; rows 4 I0 .. 4 I1 - 1 of this thread's
+    auto mul = [&](auto sub, auto lo, auto hi, int s, int kb) {
+        constexpr bool SUB = decltype(sub)::value;
+        constexpr int I0 = 4 * decltype(lo)::value, I1 = 4 * decltype(hi)::value;
+        const float *A = ring + (s & 1) * PIECE + 4 * ty, *B = sX + kb * LDX + 4 * tx;
+#pragma unroll 2
+        for (int k = 0; k < PK; k++) {
+            float a[8], b[8];
+            if (I0 == 0) ld4(a, A + k * KB);
+            if (I1 == 8) ld4(a + 4, A + k * KB + 32);
+            ld4(b, B + k * LDX);
+            ld4(b + 4, B + k * LDX + NC);
+#pragma unroll
+            for (int i = I0; i < I1; i++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[i][j] = SUB ? fmaf(-a[i], b[j], acc[i][j]) : fmaf(a[i], b[j], acc[i][j]);
+        }
+    };
+    using C0 = std::integral_constant<int, 0>;
+    using C1 = std::integral_constant<int, 1>;
+    using C2 = std::integral_constant<int, 2>;
+    bool tmo = false;
+    start(0);
+    __syncthreads();
+#pragma unroll 1
+    for (int s = 0; s < 8 * cnt; s++) {
+        const int q = s & 3;
+        tmo |= !mbar_wait(bars + (s & 1), (unsigned)(s >> 1) & 1u);
+        if (s & 4) {
+            mul(std::false_type(), C0(), C2(), s, q * PK);
+        } else { // T = Z - E X; E is lower triangular at the top, upper at the bottom
+            const bool lo = top ? q <= w : q >= w, hi = top ? q <= w + 2 : q >= w + 2; // rows 16 w .. and 32 + 16 w ..
+            if (lo && hi)
+                mul(std::true_type(), C0(), C2(), s, q * PK);
+            else if (lo)
+                mul(std::true_type(), C0(), C1(), s, q * PK);
+            else if (hi)
+                mul(std::true_type(), C1(), C2(), s, q * PK);
+        }
+        if (__syncthreads_or(tmo)) { // every thread has used the piece (and X's rows)
+            if (threadIdx.x == 0) atomicOr(err, SPK_DEV_ERR_TIMEOUT);
+            if (s + 1 < 8 * cnt) mbar_wait(bars + ((s + 1) & 1), (unsigned)((s + 1) >> 1) & 1u);
+            return;
+        }
+        issue(s + 2);
+        if (q == 3) { // T, then X_J
+            if (s & 4)
+                asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); // Z_J has been read by both
+            else
+                asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                st4(sX + row(i) * LDX + 4 * tx, acc[i]);
+                st4(sX + row(i) * LDX + NC + 4 * tx, acc[i] + 4);
+            }
+            if (s & 4) {
+                const size_t x = tb + (size_t)block(s >> 3) * TS + (size_t)(cb + 4 * tx) * KB + 4 * ty; // column-major
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+#pragma unroll
+                    for (int i = 0; i < 8; i += 4) {
+                        const float v[4] = {acc[i][j], acc[i + 1][j], acc[i + 2][j], acc[i + 3][j]};
+                        if (j < 4 ? doV : doW) st4((j < 4 ? gV : gW) + x + (j & 3) * KB + 8 * i, v);
+                    }
+                start((s >> 3) + 1);
+            } else {
+#pragma unroll
+                for (int a = 0; a < 8; a++)
+#pragma unroll
+                    for (int j = 0; j < 8; j++) acc[a][j] = 0.f;
+            }
+            __syncthreads();
+        }
+    }
+}
+
 // ------------------------------------------------------------ small bands
 // KB <= 4: the same two-sided recurrences on KB lanes per chain (lane r owns
 // row r of every tile; the other rows arrive by shuffles), with each chain's
@@ -1032,9 +1191,13 @@ template <class T, int KB> int run_twist(spk_plan *P, cudaStream_t st, bool fwd,
                     cudaSuccess ||
                 cudaFuncSetAttribute(k_tw_merge<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem) !=
                     cudaSuccess ||
-                cudaFuncSetAttribute(k_tw_bwd<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem) !=
+                cudaFuncSetAttribute(k_tw_bwd_vw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TwVW::SMEM) !=
                     cudaSuccess)
                 return SPK_ECUDA;
+            if constexpr (!TwCfg<T, KB>::T88)
+                if (cudaFuncSetAttribute(k_tw_bwd<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem) !=
+                    cudaSuccess)
+                    return SPK_ECUDA;
             if constexpr (tw_lu_w_ok<T, KB>()) {
                 if (cudaFuncSetAttribute(k_tw_lu_w<T, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)tw_lu_w_smem<T, KB>()) != cudaSuccess ||
@@ -1078,15 +1241,21 @@ template <class T, int KB> int run_twist(spk_plan *P, cudaStream_t st, bool fwd,
             SPK_CHECK_LAUNCH();
             P->launches++;
         } else if (p > 1) {
+            int rc = SPK_OK;
             if constexpr (tw_lu_w_ok<T, KB>())
                 k_tw_bwd_w<T, KB><<<(4 * np + TW_W_CHAINS - 1) / TW_W_CHAINS, 32 * TW_W_CHAINS,
                                     tw_lu_w_smem<T, KB>(), st>>>(P->d_blk_off, p, (const T *)P->d_G,
                                                                  (const T *)P->d_E, (T *)P->d_V, (T *)P->d_W, part0,
                                                                  np, P->d_err);
+            else if constexpr (TwCfg<T, KB>::T88)
+                rc = launch_dep(k_tw_bwd_vw, dim3(2 * np, 2), TwVW::NT, TwVW::SMEM, 2, false, st, (const int *)P->d_blk_off,
+                                p, (const float *)P->d_G, (const float *)P->d_E, (float *)P->d_V, (float *)P->d_W, part0,
+                                P->d_err);
             else
                 k_tw_bwd<T, KB><<<dim3(np, 4), NT, C::smem, st>>>(P->d_blk_off, p, (const T *)P->d_G,
                                                                   (const T *)P->d_E, (T *)P->d_V, (T *)P->d_W, part0,
                                                                   P->d_err);
+            if (rc != SPK_OK) return rc;
             SPK_CHECK_LAUNCH();
             P->launches++;
         }
