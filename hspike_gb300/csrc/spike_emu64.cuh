@@ -73,19 +73,7 @@ template <int KB> struct Emu {
         constexpr int ST = KB * LDP / 2;
 #pragma unroll
         for (int i = 0; i < K / 8; i++) {
-            unsigned a0, b0, m0, a1, b1, m1;
-            sl_split(live ? v[i][0] : 0.0, live ? E : 64, a0, b0, m0);
-            sl_split(live ? v[i][1] : 0.0, live ? E : 64, a1, b1, m1);
-            unsigned *p = o + 4 * i;
-            p[0] = sl_digit<0>(a0, b0, a1, b1);
-            p[ST] = sl_digit<1>(a0, b0, a1, b1);
-            p[2 * ST] = sl_digit<2>(a0, b0, a1, b1);
-            p[3 * ST] = sl_digit<3>(a0, b0, a1, b1);
-            p[4 * ST] = sl_digit<4>(a0, b0, a1, b1);
-            p[5 * ST] = sl_digit<5>(a0, b0, a1, b1);
-            p[6 * ST] = sl_digit<6>(a0, b0, a1, b1);
-            p[7 * ST] = sl_digit<7>(a0, b0, a1, b1);
-            p[8 * ST] = m0 | (m1 << 16);
+            SlPair(live ? v[i][0] : 0.0, live ? v[i][1] : 0.0, live ? E : 64).store(o + 4 * i, ST);
         }
     }
 

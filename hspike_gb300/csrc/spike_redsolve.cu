@@ -802,20 +802,8 @@ __global__ void __launch_bounds__(RedSl<KB>::NT)
         const int x = warp + w * Q::WARPS, h = x / (Q::K / 64), k = x % (Q::K / 64) * 64 + 2 * lane;
         const int E = ec[h];
         const bool live = E >= 64 && E < 0x7ff;
-        unsigned a0, b0, m0, a1, b1, m1;
-        sl_split(live ? v[w][0] : 0.0, live ? E : 64, a0, b0, m0);
-        sl_split(live ? v[w][1] : 0.0, live ? E : 64, a1, b1, m1);
-        unsigned *o = (unsigned *)(px + h * Q::LDX + k);
-        constexpr int ST = Q::NC * Q::LDX / 2;
-        o[0] = sl_digit<0>(a0, b0, a1, b1);
-        o[ST] = sl_digit<1>(a0, b0, a1, b1);
-        o[2 * ST] = sl_digit<2>(a0, b0, a1, b1);
-        o[3 * ST] = sl_digit<3>(a0, b0, a1, b1);
-        o[4 * ST] = sl_digit<4>(a0, b0, a1, b1);
-        o[5 * ST] = sl_digit<5>(a0, b0, a1, b1);
-        o[6 * ST] = sl_digit<6>(a0, b0, a1, b1);
-        o[7 * ST] = sl_digit<7>(a0, b0, a1, b1);
-        o[8 * ST] = m0 | (m1 << 16);
+        SlPair(live ? v[w][0] : 0.0, live ? v[w][1] : 0.0, live ? E : 64)
+            .store((unsigned *)(px + h * Q::LDX + k), Q::NC * Q::LDX / 2);
     }
     __syncthreads();
     SlAcc acc;

@@ -5,7 +5,7 @@
 // (2 multiply-adds per clock and SM) is what bounds it from two columns on:
 // n = 2,000,000, k = 64, 16 columns took 8.93 ms a pass, 75 % of that pipe's
 // rate, where reading the 2.1 GB of values takes 0.31 ms.  Here a warp forms 16
-// rows x 8 columns at a time by exact FP16 digit products: 2.55 ms.
+// rows x 8 columns at a time by exact FP16 digit products: 2.35 ms.
 //
 // A full band -- its entry count says so, since the columns of a row are
 // distinct and within the band -- has row r's entries in columns
@@ -175,20 +175,8 @@ __global__ void __launch_bounds__(32 * NW * KS, 2)
             if (h < NC) {
                 const int E = ec[h];
                 const bool live = E >= 64 && E < 0x7ff;
-                unsigned a0, b0, m0, a1, b1, m1;
-                sl_split(live ? v[u][0] : 0.0, live ? E : 64, a0, b0, m0);
-                sl_split(live ? v[u][1] : 0.0, live ? E : 64, a1, b1, m1);
-                unsigned *o = (unsigned *)(px + (size_t)h * G.ldx + k);
-                const int st = NC * G.ldx / 2;
-                o[0] = sl_digit<0>(a0, b0, a1, b1);
-                o[st] = sl_digit<1>(a0, b0, a1, b1);
-                o[2 * st] = sl_digit<2>(a0, b0, a1, b1);
-                o[3 * st] = sl_digit<3>(a0, b0, a1, b1);
-                o[4 * st] = sl_digit<4>(a0, b0, a1, b1);
-                o[5 * st] = sl_digit<5>(a0, b0, a1, b1);
-                o[6 * st] = sl_digit<6>(a0, b0, a1, b1);
-                o[7 * st] = sl_digit<7>(a0, b0, a1, b1);
-                o[8 * st] = m0 | (m1 << 16);
+                SlPair(live ? v[u][0] : 0.0, live ? v[u][1] : 0.0, live ? E : 64)
+                    .store((unsigned *)(px + (size_t)h * G.ldx + k), NC * G.ldx / 2);
             }
         }
         __syncthreads();

@@ -32,7 +32,7 @@ constexpr float SL_GUARD = 0.015625f; // 2^-6 (the magnitudes are rounded down t
 // biased exponent of |v| (0 for zero and subnormals, 0x7ff for inf and NaN)
 __device__ __forceinline__ int sl_exp(double v) { return (int)(((unsigned)__double2hiint(v) >> 20) & 0x7ffu); }
 
-// the 64-bit word whose bytes are the digits of v (+128 each) at scale exponent
+// the 64-bit word whose bytes are the digits of |v| (+128 each) at scale exponent
 // E (biased; every value of the row has exponent <= E, 64 <= E < 0x7ff; a zero
 // or subnormal v shifts out whole), and |v| 2^-E rounded down to a power of two, in FP16
 __device__ __forceinline__ void sl_split(double v, int E, unsigned &hi, unsigned &lo, unsigned &mag)
@@ -43,24 +43,56 @@ __device__ __forceinline__ void sl_split(double v, int E, unsigned &hi, unsigned
     const unsigned mh = __funnelshift_l(vl, (vh & 0xfffffu) | 0x100000u, 9), ml = vl << 9;
     unsigned long long m = ((unsigned long long)mh << 32) | ml, q;
     asm("shr.u64 %0, %1, %2;" : "=l"(q) : "l"(m), "r"(sh)); // shifts of 64 and more give 0
-    const long long sg = (long long)((int)vh >> 31);
-    m = (unsigned long long)(((long long)q ^ sg) - sg) + 0x8080808080808080ull;
+    m = q + 0x8080808080808080ull;
     hi = (unsigned)(m >> 32);
     lo = (unsigned)m;
     mag = (unsigned)max(15 - (int)sh, 0) << 10;
 }
 
-// digit I (0 = leading) of two values packed as FP16: low half from (hi0, lo0)
-template <int I>
-__device__ __forceinline__ unsigned sl_digit(unsigned hi0, unsigned lo0, unsigned hi1, unsigned lo1)
-{
-    constexpr int B = 3 - (I & 3); // byte within the word
-    const unsigned a = I < 4 ? hi0 : lo0, b = I < 4 ? hi1 : lo1;
-    // bytes a.B and b.B under the exponent of 1024: 1024 + u, exact; then u - 128
-    const unsigned p = (__byte_perm(a, b, B | (B << 4) | ((4 + B) << 8) | ((4 + B) << 12)) & 0x00ff00ffu) | 0x64006400u;
-    const __half2 d = __hsub2(*reinterpret_cast<const __half2 *>(&p), __float2half2_rn(1152.f));
-    return *reinterpret_cast<const unsigned *>(&d);
-}
+// Two values of one row (or column), their digits packed as FP16 pairs on
+// demand.  A digit's bytes under the exponent of 1024 are 1024 + 128 + d, exact,
+// and one fused multiply-add takes the bias off and puts the sign on: d is a
+// digit of |v|, which spares negating the 64-bit words.
+struct SlPair {
+    unsigned q[4];      // bytes of digits 2 i (v0, v1), 2 i + 1 (v0, v1)
+    unsigned sg, nb;    // +-1 and -+1152 of both signs
+    unsigned mg;        // the magnitudes
+    __device__ __forceinline__ SlPair(double v0, double v1, int E)
+    {
+        unsigned h0, l0, m0, h1, l1, m1;
+        sl_split(v0, E, h0, l0, m0);
+        sl_split(v1, E, h1, l1, m1);
+        q[0] = __byte_perm(h0, h1, 0x6273);
+        q[1] = __byte_perm(h0, h1, 0x4051);
+        q[2] = __byte_perm(l0, l1, 0x6273);
+        q[3] = __byte_perm(l0, l1, 0x4051);
+        const unsigned s = __byte_perm((unsigned)__double2hiint(v0), (unsigned)__double2hiint(v1), 0x7030) & 0x80008000u;
+        sg = s | 0x3c003c00u;
+        nb = s ^ 0xe480e480u;
+        mg = m0 | (m1 << 16);
+    }
+    // digit I (0 = leading): low half of v0, high half of v1
+    template <int I> __device__ __forceinline__ unsigned digit() const
+    {
+        const unsigned p = __byte_perm(q[I / 2], 0x64646464u, I & 1 ? 0x4342 : 0x4140);
+        const __half2 d = __hfma2(*reinterpret_cast<const __half2 *>(&p), *reinterpret_cast<const __half2 *>(&sg),
+                                  *reinterpret_cast<const __half2 *>(&nb));
+        return *reinterpret_cast<const unsigned *>(&d);
+    }
+    // all digits and the magnitudes, st words apart
+    __device__ __forceinline__ void store(unsigned *o, int st) const
+    {
+        o[0] = digit<0>();
+        o[st] = digit<1>();
+        o[2 * st] = digit<2>();
+        o[3 * st] = digit<3>();
+        o[4 * st] = digit<4>();
+        o[5 * st] = digit<5>();
+        o[6 * st] = digit<6>();
+        o[7 * st] = digit<7>();
+        o[8 * st] = mg;
+    }
+};
 
 __device__ __forceinline__ void sl_mma(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1)
 {
@@ -80,19 +112,17 @@ struct SlFragA {
         for (int r = 0; r < 2; r++)
 #pragma unroll
             for (int q = 0; q < 2; q++) {
-                unsigned h0, l0, m0, h1, l1, m1;
-                sl_split(v[r][2 * q], r ? E1 : E0, h0, l0, m0);
-                sl_split(v[r][2 * q + 1], r ? E1 : E0, h1, l1, m1);
+                const SlPair d(v[r][2 * q], v[r][2 * q + 1], r ? E1 : E0);
                 const int f = r + 2 * q; // fragment registers: (g, lo), (g + 8, lo), (g, hi), (g + 8, hi)
-                a[0][f] = sl_digit<0>(h0, l0, h1, l1);
-                a[1][f] = sl_digit<1>(h0, l0, h1, l1);
-                a[2][f] = sl_digit<2>(h0, l0, h1, l1);
-                a[3][f] = sl_digit<3>(h0, l0, h1, l1);
-                a[4][f] = sl_digit<4>(h0, l0, h1, l1);
-                a[5][f] = sl_digit<5>(h0, l0, h1, l1);
-                a[6][f] = sl_digit<6>(h0, l0, h1, l1);
-                a[7][f] = sl_digit<7>(h0, l0, h1, l1);
-                mg[f] = m0 | (m1 << 16);
+                a[0][f] = d.digit<0>();
+                a[1][f] = d.digit<1>();
+                a[2][f] = d.digit<2>();
+                a[3][f] = d.digit<3>();
+                a[4][f] = d.digit<4>();
+                a[5][f] = d.digit<5>();
+                a[6][f] = d.digit<6>();
+                a[7][f] = d.digit<7>();
+                mg[f] = d.mg;
             }
     }
 };
