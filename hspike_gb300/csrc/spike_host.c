@@ -312,7 +312,41 @@ int spk_choose_block(int k)
  * must hold at least two tiles (2 KB rows) so that its top and bottom tips
  * are distinct; a requested p is clamped to that, an automatic p fills the
  * GPU: two CTAs per SM for the large tiles, more for the small ones. */
-static int choose_partitions(int n, int KB, int requested)
+/* An automatic count of tiles of 32 rows and more, where n does not give every
+ * SM its chains (fewer than 8 tiles each, 4 of 128 rows: the partitions would not
+ * be eliminated from both ends either).  The time is then latency: tiles one after
+ * the other in a chain, and levels of the reduced system, each of which costs
+ * as much as one or two tiles and more the more blocks its first ones have.  A
+ * level takes 2^L interfaces as well as fewer, so the counts to weigh are 2^L + 1.
+ * Two tiles per partition (the most partitions there can be) against the choice:
+ * n = 20,000, k = 48, 16 columns 1,009 / 879 us (156, 33 partitions), one column
+ * 694 / 630; n = 80,000, k = 64 1,037 / 942 (304, 129); n = 2,000, k = 64 403 / 392
+ * (15, 9); n = 40,000, k = 24 601 / 498 (304, 129); n = 3,000, k = 24 374 / 344 (46, 9);
+ * n = 33,000, k = 100, 8 columns 1,921 / 1,771 (128, 65).  Smaller tiles keep the
+ * most: their levels are cheap (n = 5,000, k = 8 211 / 246 with four tiles each),
+ * and so do complex tiles of 64 rows, whose chains are dear (n = 10,000, k = 60
+ * 1,121 / 1,371 with 17 partitions). */
+static int fewer_partitions(int n, int KB, int pmax)
+{
+    const double level = KB >= 128 ? 0.95 : KB == 64 ? 1.7 : 2.5; /* tiles' worth of a level */
+    const double both = KB >= 128 ? 1.0 : KB == 64 ? 0.7 : 0.5;   /* of a tile eliminated from both ends */
+    int best = pmax;
+    double cost = 1e30;
+    for (int L = 0; L < 31; L++) {
+        int p = (1 << L) + 1;
+        if (p > pmax) p = pmax;
+        const int rows = (n + p - 1) / p, tiles = (rows + KB - 1) / KB;
+        const double c = (tiles >= 8 ? both : 1.0) * tiles + level * L * (1.0 + p / 300.0);
+        if (c < cost) {
+            cost = c;
+            best = p;
+        }
+        if (p == pmax) break;
+    }
+    return best;
+}
+
+static int choose_partitions(int n, int KB, int requested, int is_complex)
 {
     long long pmax = n / (2LL * KB);
     if (pmax < 1) pmax = 1;
@@ -322,6 +356,8 @@ static int choose_partitions(int n, int KB, int requested)
         if (sms <= 0) sms = 152;
         const int per_sm = KB >= 128 ? 1 : KB >= 32 ? 2 : KB == 16 ? 8 : 16;
         p = (long long)sms * per_sm;
+        if (KB >= 32 && !(is_complex && KB >= 64) && pmax >= 2 && n < (KB >= 128 ? 4LL : 8LL) * KB * p)
+            return fewer_partitions(n, KB, (int)(p < pmax ? p : pmax));
     }
     if (p > pmax) p = pmax;
     if (p < 1) p = 1;
@@ -341,7 +377,7 @@ static int choose_partitions(int n, int KB, int requested)
 static int subdivision(int n, int KB, int requested, int p)
 {
     if (requested <= 0) return 1;
-    int target = choose_partitions(1 << 30, KB, 0); /* what fills the GPU */
+    int target = choose_partitions(1 << 30, KB, 0, 0); /* what fills the GPU */
     if (KB <= 4 && target > 2048) target = 2048;
     const long long most = (n / p) / ((KB >= 64 ? 8LL : 16LL) * KB);
     const long long sub = target / p < most ? target / p : most;
@@ -569,7 +605,7 @@ static int plan_create(int n, long long nnz, int ku, int kl, int is_complex, int
     const int k = ku > kl ? ku : kl;
     const int KB = spk_choose_block(k < 1 ? 1 : k);
     if (!KB || spk_factor_smem(KB, is_complex, mode) == 0) return SPK_EBAND;
-    const int p = choose_partitions(n, KB, partitions), sub = subdivision(n, KB, partitions, p);
+    const int p = choose_partitions(n, KB, partitions, is_complex), sub = subdivision(n, KB, partitions, p);
     int *ps = (int *)malloc(sizeof(int) * ((size_t)p * sub + 1));
     if (!ps) return SPK_EMEM;
     /* A partition count the caller asked for gets the reference's layout
@@ -595,7 +631,7 @@ size_t spk_solve_footprint(int n, long long nnz, int k, int nrhs, int is_complex
 {
     const int KB = spk_choose_block(k < 1 ? 1 : k);
     if (!KB || n <= 0) return 0;
-    int p = choose_partitions(n, KB, partitions);
+    int p = choose_partitions(n, KB, partitions, is_complex);
     const int nreg = n / p, sub = subdivision(n, KB, partitions, p);
     /* blocks of m rows in `pieces` balanced pieces: m % pieces of them hold one row more */
 #define PIECES(m, pieces)                                                                                       \
@@ -643,7 +679,7 @@ static int plan_matches(const spk_plan *P, int n, int ku, int kl, int is_complex
     const int k = ku > kl ? ku : kl;
     const int KB = spk_choose_block(k < 1 ? 1 : k);
     return P->n == n && P->KB == KB && P->is_complex == is_complex && P->mode == mode &&
-           P->p_user == choose_partitions(n, KB, partitions) &&
+           P->p_user == choose_partitions(n, KB, partitions, is_complex) &&
            P->p == P->p_user * subdivision(n, KB, partitions, P->p_user) && nrhs <= P->nrhs_max;
 }
 
@@ -821,7 +857,7 @@ static int run_device(spike_context_t c, int n, long long nnz, int nrhs, const i
      * call fall back to analysis, a new plan and a second factorization. */
     spk_plan *Q = c->plan;
     if (Q && Q->n == n && Q->nnz == nnz && Q->is_complex == is_complex && Q->mode == c->mode &&
-        Q->p_user == choose_partitions(n, Q->KB, c->partitions) &&
+        Q->p_user == choose_partitions(n, Q->KB, c->partitions, is_complex) &&
         Q->p == Q->p_user * subdivision(n, Q->KB, c->partitions, Q->p_user) && chunk0 <= Q->nrhs_max) {
         unsigned e[4];
         Q->twist = Q->twist_cap && c->twist;
@@ -1045,7 +1081,7 @@ static int host_pipelined(spike_context_t c, int n, long long nnz, int nrhs, con
     spk_plan *Q = c->plan;
     const int chunk = nrhs < RHS_CHUNK ? nrhs : RHS_CHUNK;
     if (!Q || Q->n != n || Q->nnz != nnz || Q->is_complex != cplx || Q->mode != c->mode || !Q->twist_cap || !c->twist ||
-        Q->p_user != choose_partitions(n, Q->KB, c->partitions) ||
+        Q->p_user != choose_partitions(n, Q->KB, c->partitions, cplx) ||
         Q->p != Q->p_user * subdivision(n, Q->KB, c->partitions, Q->p_user) || chunk > Q->nrhs_max ||
         Q->p < PIPE_RANGES ||
         Q->KB < 16 || Q->KB > 64 ||
@@ -1545,7 +1581,7 @@ Error_t spike_dsolve_device_noalloc(integer_t n, integer_t nnz, integer_t nrhs, 
     const int KB = spk_choose_block(k < 1 ? 1 : k);
     if (!KB || spk_factor_smem(KB, 0, SPK_MIXED) == 0)
         return spk_fail(SPIKE_ERR_BANDWIDTH, "%s: bandwidth %d above the supported tile size", name, k);
-    int p = choose_partitions(n, KB, 0);
+    int p = choose_partitions(n, KB, 0, 0);
     if (p > NOALLOC_MAX_PARTS) p = NOALLOC_MAX_PARTS;
     int part_start[NOALLOC_MAX_PARTS + 1], blk_off[NOALLOC_MAX_PARTS + 1];
     int cr_count[32];
