@@ -1256,11 +1256,11 @@ __global__ void __launch_bounds__(256)
 // on neighbouring lanes, so they share each load of the row's spike entries:
 // the spikes cross from DRAM once, not once per column (at 4-row complex
 // tiles and 4 million rows they are 256 MB, twice the L2).
-template <class T, int KB>
+template <class T, int KB, class U>
 __global__ void __launch_bounds__(256)
     k_retrieve_rc(const int *__restrict__ part_start, const int *__restrict__ blk_off, int p,
                     const int *__restrict__ blk_part, const T *__restrict__ gV, const T *__restrict__ gW,
-                    const T *__restrict__ gy, const typename HighOf<T>::type *__restrict__ u, long long NP, int n_iface, int n, int nrhs,
+                    const T *__restrict__ gy, const U *__restrict__ u, long long NP, int n_iface, int n, int nrhs,
                     typename HighOf<T>::type *x, int accumulate, const spk_sysref *__restrict__ sys,
                     const int *__restrict__ part_sys)
 {
@@ -1268,6 +1268,12 @@ __global__ void __launch_bounds__(256)
     dep_launch();
     dep_wait();
     constexpr size_t TS = (size_t)KB * KB;
+    auto val = [](U v) -> T {
+        if constexpr (std::is_same<T, U>::value)
+            return v;
+        else
+            return cvt_fast<T, U>(v);
+    };
     const long long NR = (long long)n_iface * 2 * KB;
     const long long tot = NP * nrhs;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < tot;
@@ -1289,14 +1295,14 @@ __global__ void __launch_bounds__(256)
         }
         T acc = gy[(size_t)h * NP + pr];
         if (part < p - 1) {
-            const H *t = u + (size_t)h * NR + (size_t)part * 2 * KB + KB;
+            const U *t = u + (size_t)h * NR + (size_t)part * 2 * KB + KB;
 #pragma unroll
-            for (int c = 0; c < KB; c++) acc = msub(acc, gV[(size_t)gb * TS + (size_t)c * KB + lr], cvt_fast<T, H>(t[c]));
+            for (int c = 0; c < KB; c++) acc = msub(acc, gV[(size_t)gb * TS + (size_t)c * KB + lr], val(t[c]));
         }
         if (part > 0) {
-            const H *bw = u + (size_t)h * NR + (size_t)(part - 1) * 2 * KB;
+            const U *bw = u + (size_t)h * NR + (size_t)(part - 1) * 2 * KB;
 #pragma unroll
-            for (int c = 0; c < KB; c++) acc = msub(acc, gW[(size_t)gb * TS + (size_t)c * KB + lr], cvt_fast<T, H>(bw[c]));
+            for (int c = 0; c < KB; c++) acc = msub(acc, gW[(size_t)gb * TS + (size_t)c * KB + lr], val(bw[c]));
         }
         H *xp = xb + (size_t)h * ld + s + lrow;
         const H d = cvt_fast<H, T>(acc);
@@ -1396,15 +1402,17 @@ template <class T, int KB> int run_retrieve(spk_plan *P, void *x, int nrhs, int 
 {
     using H = typename HighOf<T>::type;
     // the interface unknowns, narrowed once into the (now free) reduced-RHS work
-    // array; rows of up to four unknowns per spike convert their own, and plain
-    // precision has nothing to narrow.  Each launch may start while the one before
-    // runs out (n = 1,000, k = 2: 172 -> 154 us a solve with that and without the
-    // narrowing), but not in a batch, where waiting CTAs take another group's place
-    // (512 systems: 8.2 ms against 8.0).
-    constexpr bool NARROW = KB > 4 && !std::is_same<T, H>::value;
-    T *ut = NARROW ? (T *)P->d_crg : (T *)P->d_u;
+    // array.  Plain precision has nothing to narrow, and rows of up to four
+    // unknowns per spike convert their own where they are few: n = 1,000, k = 2
+    // saves a launch of 3 us, n = 4,000,000, k = 3, complex, four columns would pay 330 us
+    // a pass.  Each launch may start while the one before runs out (that and the
+    // narrowing: 172 -> 150 us for the small solve), but not in a batch, where
+    // waiting CTAs take another group's place (512 systems: 8.2 ms against 8.0).
+    constexpr bool SAME = std::is_same<T, H>::value;
+    const bool own = KB <= 4 && P->NP * nrhs <= 1 << 16, narrow = !SAME && !own;
+    T *ut = SAME ? (T *)P->d_u : (T *)P->d_crg;
     const long long cnt = (long long)(P->n_iface > 0 ? P->n_iface : 1) * 2 * KB * nrhs;
-    if (NARROW && P->n_iface > 0) {
+    if (narrow && P->n_iface > 0) {
         if (launch_dep(k_u_narrow<T>, dim3((unsigned)std::min<long long>((cnt + 255) / 256, 4096)), 256, 0, 1, !P->d_sys, st,
                        (const H *)P->d_u, ut, cnt) != SPK_OK)
             return SPK_ECUDA;
@@ -1418,10 +1426,13 @@ template <class T, int KB> int run_retrieve(spk_plan *P, void *x, int nrhs, int 
         if constexpr (KB <= 4) {
             const long long tot = P->NP * nrhs;
             const int grid = (int)std::min<long long>((tot + 255) / 256, (long long)cap);
-            if (launch_dep(k_retrieve_rc<T, KB>, dim3(grid), 256, 0, 1, !P->d_sys, st, (const int *)P->d_part_start,
-                           (const int *)P->d_blk_off, P->p, (const int *)P->d_blk_part, (const T *)P->d_V,
-                           (const T *)P->d_W, (const T *)P->d_y, (const H *)P->d_u, P->NP, P->n_iface, P->n, nrhs, (H *)x,
-                           accumulate, (const spk_sysref *)P->d_sys, (const int *)P->d_part_sys) != SPK_OK)
+            auto go = [&](auto kern, auto *u) {
+                return launch_dep(kern, dim3(grid), 256, 0, 1, !P->d_sys, st, (const int *)P->d_part_start,
+                                  (const int *)P->d_blk_off, P->p, (const int *)P->d_blk_part, (const T *)P->d_V,
+                                  (const T *)P->d_W, (const T *)P->d_y, u, P->NP, P->n_iface, P->n, nrhs, (H *)x,
+                                  accumulate, (const spk_sysref *)P->d_sys, (const int *)P->d_part_sys);
+            };
+            if ((own ? go(k_retrieve_rc<T, KB, H>, (const H *)P->d_u) : go(k_retrieve_rc<T, KB, T>, (const T *)ut)) != SPK_OK)
                 return SPK_ECUDA;
         } else {
             const long long tot = P->NP * ((nrhs + RET_HC - 1) / RET_HC);

@@ -1524,9 +1524,14 @@ __device__ __forceinline__ float f64_to_f32_try(double x, bool &rare)
 }
 __device__ __forceinline__ float f64_to_f32(double x)
 {
-    bool rare = false;
-    const float f = f64_to_f32_try(x, rare);
-    return rare ? f64_to_f32_rare(x) : f;
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int e = (int)((hi >> 20) & 0x7ffu) - 1023 + 127;
+    if (e <= 0 || e >= 255) return f64_to_f32_rare(x);
+    const unsigned r = ((hi & 0xfffffu) << 3) | (lo >> 29); // 23 mantissa bits
+    const unsigned rem = lo & 0x1fffffffu;                  // 29 dropped bits
+    const unsigned up = (rem > 0x10000000u) || (rem == 0x10000000u && (r & 1u));
+    // a carry out of the mantissa bumps the exponent (to inf at the top), as it should
+    return __uint_as_float(((hi & 0x80000000u) | ((unsigned)e << 23)) + r + up);
 }
 // FP32 -> FP64 (exact) with integer instructions, for the same reason.  Normal
 // inputs only; zero, subnormal, inf and NaN take the hardware conversion.
