@@ -32,7 +32,7 @@ constexpr int RCS = RC + 1; // row stride of the shared [KB][RC] vectors (odd: c
 // Four or more columns: each thread accumulates a 4 x 4 block (4 rows of M
 // by one 16-byte load, 4 columns of v) over a slice of k, so a step moves
 // 0.5 shared-memory words per FMA instead of 2; the k slices of a block are
-// summed by shuffles.  Fewer columns: one output per lane group, k split
+// summed by a transposing exchange.  Fewer columns: one output per lane group, k split
 // across the group.
 template <class T, int KB, bool HAS_BASE, int S = RCS>
 __device__ void tile_mv(T *out, const T *Mt, const T *v, const T *base, int nr, bool negate)
@@ -72,23 +72,49 @@ __device__ void tile_mv(T *out, const T *Mt, const T *v, const T *base, int nr, 
 #pragma unroll
                     for (int c = 0; c < 4; c++) acc[i][c] = madd(acc[i][c], m[i], w[c]);
             }
-            for (int off = spl >> 1; off > 0; off >>= 1)
+            // the slices' sums, each lane of a group ending with its share of the
+            // 16 results (12 shuffles instead of 32 at four slices)
+            auto put = [&](auto spl_c) {
+                constexpr int SPL = decltype(spl_c)::value;
+                T f[16];
 #pragma unroll
-                for (int i = 0; i < 4; i++)
+                for (int e = 0; e < 16; e++) f[e] = acc[e / 4][e % 4];
+                auto exchange = [&](auto off_c, auto n_c) {
+                    constexpr int off = decltype(off_c)::value, n = decltype(n_c)::value;
+                    const bool up = (part & off) != 0;
 #pragma unroll
-                    for (int c = 0; c < 4; c++) acc[i][c] = acc[i][c] + shfl_xor_any(acc[i][c], off);
-            if (valid && part == 0) {
+                    for (int e = 0; e < n; e++) {
+                        const T send = up ? f[e] : f[e + n];
+                        f[e] = (up ? f[e + n] : f[e]) + shfl_xor_any(send, off);
+                    }
+                };
+                using C1 = std::integral_constant<int, 1>;
+                using C2 = std::integral_constant<int, 2>;
+                using C4 = std::integral_constant<int, 4>;
+                using C8 = std::integral_constant<int, 8>;
+                if constexpr (SPL == 8) exchange(C4(), C8()), exchange(C2(), C4()), exchange(C1(), C2());
+                if constexpr (SPL == 4) exchange(C2(), C8()), exchange(C1(), C4());
+                if constexpr (SPL == 2) exchange(C1(), C8());
+                if (!valid) return;
 #pragma unroll
-                for (int i = 0; i < 4; i++)
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        if (h0 + c < nr) {
-                            const int q = (r0 + i) * S + h0 + c;
-                            T val = negate ? -acc[i][c] : acc[i][c];
-                            if (HAS_BASE) val = base[q] + val;
-                            out[q] = val;
-                        }
-            }
+                for (int e = 0; e < 16 / SPL; e++) {
+                    const int x = part * (16 / SPL) + e, h = h0 + x % 4;
+                    if (h < nr) {
+                        const int q = (r0 + x / 4) * S + h;
+                        T val = negate ? -f[e] : f[e];
+                        if (HAS_BASE) val = base[q] + val;
+                        out[q] = val;
+                    }
+                }
+            };
+            if (spl == 8)
+                put(std::integral_constant<int, 8>());
+            else if (spl == 4)
+                put(std::integral_constant<int, 4>());
+            else if (spl == 2)
+                put(std::integral_constant<int, 2>());
+            else
+                put(std::integral_constant<int, 1>());
         }
         return;
       }
