@@ -988,7 +988,8 @@ template <class T, int KB> struct TileW {
 };
 
 // ------------------------------------------------------------ blocked inverse in shared memory
-// In-place inverse without pivoting of an N x N FP32 tile (N = 32, 64, row stride LD) in shared memory, by halves: with H11 = A11^{-1}, U = A21 H11,
+// In-place inverse without pivoting of an N x N FP32 tile (N = 32, 64, 128, row
+// stride LD) in shared memory, by halves: with H11 = A11^{-1}, U = A21 H11,
 // T = H11 A12 and H22 = (A22 - U A12)^{-1},
 //     G12 = -T H22,  G21 = -H22 U,  G11 = H11 - G12 U.
 // The 32-row leaves are one warp's Gauss-Jordan on shuffles (TileW, rows scaled
@@ -996,8 +997,9 @@ template <class T, int KB> struct TileW {
 // where a blocked Gauss-Jordan over the whole tile pays a barrier per four
 // pivots.  One 64-row tile on an idle SM: 16,600 clocks on 64 threads, 13,400 on
 // 256, against 20,900 and 15,700; the elimination chains of n = 2,000,000, k = 64
-// (3.4 of them per SM) 2.26 -> 1.92 ms.  At 128 rows and 1,024 threads (64
-// registers each) the leaves spill and Gauss-Jordan stays faster.  All NT
+// (3.4 of them per SM) 2.26 -> 1.92 ms.  A 128-row tile takes
+// 50,600 clocks on 256 threads; Gauss-Jordan on the 1,024 threads of the 128-row
+// chains 63,400, and halves there spill (75,000).  All NT
 // threads call, the tile complete in shared memory before and after.
 // products of h x h blocks (row stride LD) on TT threads, TR x TC elements each
 template <int h, int TT, int LD> struct BlkMul {

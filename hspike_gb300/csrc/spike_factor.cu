@@ -12,14 +12,15 @@
 //
 //   k_band_tiles   (K1) CSR rows of every block -> dense factor-precision tiles
 //                  D_J, F_{J-1}^T, E_J, C^, B^; one CTA per block, in parallel.
+//                  (64-row FP64 tiles: K2 and K3 are spike_emu64.cu's.)
 //   k_factor_fwd   (K2) L_J = F_{J-1} G_{J-1},  S_J = D_J - L_J E_{J-1},
 //                  G_J = S_J^{-1} (Gauss-Jordan), and the forward sweep of the
 //                  W spike z_J = -L_J z_{J-1} (z_0 = C^_i).  Stores L, G, z.
 //   k_factor_bwd   (K3) backward sweep X_J = G_J (Z_J - E_J X_{J+1}) for
 //                  [V | W] (V's right-hand side B^_i lives in the last rows
 //                  only), storing the full spikes for explicit retrieval.
-//   k_tips         bottom/top tips of V and W into the FP64 interface blocks
-//                  of the reduced system.
+//   k_tips         bottom/top tips of V and W into the reduced system's level-0
+//                  blocks (FP64 records where a sharded solve gathers them).
 //
 // Pivot-free: A is required to be diagonally dominant enough that block
 // elimination needs no pivoting (every shipped workload is).  A zero or
