@@ -463,13 +463,16 @@ extern "C" int spk_residual(const spk_plan *P, const int *d_rowptr, const int *d
     cudaStream_t st = (cudaStream_t)stream;
     if (ck(cudaMemsetAsync(d_norms, 0, sizeof(double) * 2 * nrhs, st))) return SPK_ECUDA;
     // Digit products split every value of A once per eight columns, which pays
-    // from three columns and 128 multiply-adds a row on.  Two passes at
+    // from three columns and 112 multiply-adds a row and pass of eight on (at
+    // n = 600,000 a pass takes 115 us for any narrow band, the FP64 pipe 1.1 us per
+    // column and entry of a row: k = 7, 32 columns 1,187 / 915 us, k = 4, 32 columns
+    // 329 / 452).  Two passes at
     // n = 400,000, FP64 pipe against digits: k = 64, 8 columns 1,896 / 544 us,
     // 3 columns 1,014 / 508, 2 columns 522 / 501; k = 24, 4 columns 449 / 365,
     // 3 columns 428 / 360, 2 columns 228 / 356; k = 12, 8 columns 540 / 331,
     // 4 columns 285 / 302.
-    if (!P->is_complex && nrhs >= 3 && nrhs * (P->ku + P->kl + 1) >= 128 && P->ku <= 128 && P->kl <= 128 &&
-        full_band(P))
+    if (!P->is_complex && nrhs >= 3 && P->ku <= 128 && P->kl <= 128 &&
+        nrhs * (P->ku + P->kl + 1) >= 112 * ((nrhs + 7) / 8) && full_band(P))
         return spk_residual_slices(P, (const double *)d_aij, (const double *)d_x, (const double *)d_b, (double *)d_r, nrhs,
                                    want_bnorm, d_norms, stream);
     if (P->is_complex)
