@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(256)
     });
 }
 
-// ------------------------------------------------------------ KB <= 16: segments of several levels
+// ------------------------------------------------------------ KB <= 16 (8 in FP64): segments of several levels
 // The factorization's counterpart of the solve's segments (spike_redsolve.cu):
 // of an even block's four results P' and X' depend on its left odd neighbour
 // only, Q' and Y' on its right one, so a CTA takes a segment between two
@@ -705,7 +705,11 @@ template <class T, int KB> int run_red_factor(spk_plan *P, cudaStream_t st)
         SPK_CHECK_LAUNCH();
         P->launches += 4;
     }
-    if constexpr (KB <= 16) {
+    // (a group of 32 lanes takes a 16-row tile's FP64 products and pivots too long:
+    // n = 50,000, k = 16 1,118 us a solve in segments, 1,003 with a CTA per block and
+    // level; complex128 3,985 and 2,784)
+    constexpr bool LOW = std::is_same<T, float>::value || std::is_same<T, cfloat>::value;
+    if constexpr (KB <= 8 || (KB == 16 && LOW)) {
         return run_red_factor_s<T, KB>(P, st);
     } else if constexpr (std::is_same<T, float>::value) {
         return run_red_factor_c<KB>(P, st);
