@@ -727,39 +727,40 @@ template <class T, int KB> int run_red_factor(spk_plan *P, cudaStream_t st)
         }
         attr = true;
     }
-    auto odd = [&](const T *Pp, const T *Qp, int first, int stride, int count, T *Mo) {
+    auto odd = [&](const T *Pp, const T *Qp, int first, int stride, int count, T *Mo) -> int {
         if constexpr (EMU)
-            spk_emu_cr_odd(Pp, Qp, first, stride, count, Mo, P->d_err, st);
-        else
+            return spk_emu_cr_odd(Pp, Qp, first, stride, count, Mo, P->d_err, st);
+        else {
             k_cr_odd<T, KB><<<count, NT, S::bytes, st>>>(Pp, Qp, first, stride, Mo, P->d_err);
+            SPK_CHECK_LAUNCH();
+            return SPK_OK;
+        }
     };
     T *cP = (T *)P->d_crP, *cQ = (T *)P->d_crQ, *cX = (T *)P->d_crX, *cY = (T *)P->d_crY, *cM = (T *)P->d_crM;
+    auto even = [&](size_t o, size_t on, const T *Ml, int cnt) -> int {
+        if constexpr (EMU)
+            return spk_emu_cr_even(cP + o, cQ + o, cX + o, cY + o, Ml, cnt, cP + on, cQ + on, cX + on, cY + on, st);
+        else {
+            k_cr_even<T, KB><<<dim3((cnt + 1) / 2, 4), NT, S::bytes, st>>>(cP + o, cQ + o, cX + o, cY + o, Ml, cnt, cP + on,
+                                                                          cQ + on, cX + on, cY + on);
+            SPK_CHECK_LAUNCH();
+            return SPK_OK;
+        }
+    };
     for (int l = 0; l < P->cr_levels; l++) {
         const int cnt = P->cr_count[l];
         const size_t o = (size_t)P->cr_off[l] * TS, on = (size_t)P->cr_off[l + 1] * TS;
         T *Ml = cM + (size_t)P->cr_moff[l] * 4 * TS;
-        const int nodd = cnt / 2, neven = (cnt + 1) / 2;
-        if (nodd > 0) {
-            odd(cP + o, cQ + o, 1, 2, nodd, Ml);
-            SPK_CHECK_LAUNCH();
-        }
-        if constexpr (EMU)
-            spk_emu_cr_even(cP + o, cQ + o, cX + o, cY + o, Ml, cnt, cP + on, cQ + on, cX + on, cY + on, st);
-        else
-            k_cr_even<T, KB><<<dim3(neven, 4), NT, S::bytes, st>>>(cP + o, cQ + o, cX + o, cY + o, Ml, cnt, cP + on,
-                                                                   cQ + on, cX + on, cY + on);
-        SPK_CHECK_LAUNCH();
+        int rc = cnt / 2 > 0 ? odd(cP + o, cQ + o, 1, 2, cnt / 2, Ml) : SPK_OK;
+        if (rc == SPK_OK) rc = even(o, on, Ml, cnt);
+        if (rc != SPK_OK) return rc;
         P->launches += 2;
     }
     // top: a single block
-    {
-        const int L = P->cr_levels;
-        const size_t o = (size_t)P->cr_off[L] * TS;
-        odd(cP + o, cQ + o, 0, 1, 1, cM + (size_t)P->cr_moff[L] * 4 * TS);
-        SPK_CHECK_LAUNCH();
-        P->launches++;
-    }
-    return SPK_OK;
+    const size_t o = (size_t)P->cr_off[P->cr_levels] * TS;
+    const int rc = odd(cP + o, cQ + o, 0, 1, 1, cM + (size_t)P->cr_moff[P->cr_levels] * 4 * TS);
+    P->launches++;
+    return rc;
     }
 }
 
