@@ -1650,7 +1650,9 @@ static int launch_dep(Kern k, dim3 grid, int nt, size_t smem, int cluster, bool 
     }
     cfg.attrs = at;
     cfg.numAttrs = na;
-    return cudaLaunchKernelEx(&cfg, k, args...) == cudaSuccess ? SPK_OK : SPK_ECUDA;
+    if (cudaLaunchKernelEx(&cfg, k, args...) == cudaSuccess) return SPK_OK;
+    cudaGetLastError(); // (reported here: not to the next launch's check as well)
+    return SPK_ECUDA;
 }
 
 constexpr int RS_MAXL = 32;
