@@ -63,6 +63,7 @@ SPIKE_OPT_STREAM_ALLOC = 6
 SPIKE_OPT_TWIST = 7
 SPIKE_OPT_HOST_THREADS = 8
 SPIKE_OPT_REDUCED_FP64 = 9
+SPIKE_OPT_SPLIT_PARTITIONS = 10
 SPIKE_BATCH_AUTOTUNE = 1
 SPIKE_BATCH_NO_GRAPH = 2
 

@@ -122,6 +122,7 @@ Error_t spike_context_create(spike_context_t *out)
     c->max_refine = 3;
     c->red_refine = 0;
     c->twist = 1;
+    c->split = 1;
     c->host_threads = 8;
     c->tol = 1e-12;
     if (spk_malloc((void **)&c->d_scratch, 4 * sizeof(int)) != SPK_OK) {
@@ -223,6 +224,9 @@ Error_t spike_set_option(spike_context_t c, int opt, double v)
     case SPIKE_OPT_REDUCED_FP64:
         c->red_fp64 = v != 0;
         break;
+    case SPIKE_OPT_SPLIT_PARTITIONS:
+        c->split = v != 0;
+        break;
     case SPIKE_OPT_HOST_THREADS:
         if (v < 0 || v > 64) return spk_fail(SPIKE_ERR_ARGUMENT, "host threads must be in [0, 64]");
         c->host_threads = (int)v;
@@ -263,6 +267,7 @@ Error_t spike_get_option(spike_context_t c, int opt, double *v)
     case SPIKE_OPT_PHASE_TIMING: *v = c->timing; break;
     case SPIKE_OPT_TWIST: *v = c->twist; break;
     case SPIKE_OPT_REDUCED_FP64: *v = c->red_fp64; break;
+    case SPIKE_OPT_SPLIT_PARTITIONS: *v = c->split; break;
     case SPIKE_OPT_HOST_THREADS: *v = c->host_threads; break;
     case SPIKE_OPT_STREAM_ALLOC: *v = c->stream_alloc; break;
     default: return spk_fail(SPIKE_ERR_ARGUMENT, "unknown option %d", opt);
@@ -371,12 +376,13 @@ static int choose_partitions(int n, int KB, int requested, int is_complex)
  * does while a piece keeps at least 16 tiles (8 from 64-row tiles on), so that
  * both its halves are still eliminated at once; tiles up to 4 rows stop at the
  * 2,048 partitions that are eliminated from both ends.  The p boundaries stay
- * partition boundaries and p stays what spike_get_info reports.  With 512
+ * partition boundaries and p stays what spike_get_info reports.
+ * SPIKE_OPT_SPLIT_PARTITIONS = 0 keeps exactly p.  With 512
  * pieces each, the p = 4 solve takes 0.27 ms; 512 partitions of a complex
  * heptadiagonal n = 4,000,000 in 4 pieces each 5.49 -> 4.84 ms. */
-static int subdivision(int n, int KB, int requested, int p)
+static int subdivision(int n, int KB, int requested, int split, int p)
 {
-    if (requested <= 0) return 1;
+    if (requested <= 0 || !split) return 1;
     int target = choose_partitions(1 << 30, KB, 0, 0); /* what fills the GPU */
     if (KB <= 4 && target > 2048) target = 2048;
     const long long most = (n / p) / ((KB >= 64 ? 8LL : 16LL) * KB);
@@ -494,6 +500,7 @@ int spk_plan_build(int n, long long nnz, int ku, int kl, int KB, int is_complex,
     P->nrhs_max = nrhs_max;
     P->p = p;
     P->p_user = p;
+    P->sub = 1;
     P->n_iface = p - 1;
     P->part_start = (int *)malloc(sizeof(int) * (p + 1));
     P->blk_off = (int *)malloc(sizeof(int) * (p + 1));
@@ -598,14 +605,14 @@ int spk_plan_build(int n, long long nnz, int ku, int kl, int KB, int is_complex,
     return SPK_OK;
 }
 
-static int plan_create(int n, long long nnz, int ku, int kl, int is_complex, int mode, int partitions,
+static int plan_create(int n, long long nnz, int ku, int kl, int is_complex, int mode, int partitions, int split,
                        int nrhs_max, void *stream, int stream_alloc, spk_plan **out)
 {
     *out = NULL;
     const int k = ku > kl ? ku : kl;
     const int KB = spk_choose_block(k < 1 ? 1 : k);
     if (!KB || spk_factor_smem(KB, is_complex, mode) == 0) return SPK_EBAND;
-    const int p = choose_partitions(n, KB, partitions, is_complex), sub = subdivision(n, KB, partitions, p);
+    const int p = choose_partitions(n, KB, partitions, is_complex), sub = subdivision(n, KB, partitions, split, p);
     int *ps = (int *)malloc(sizeof(int) * ((size_t)p * sub + 1));
     if (!ps) return SPK_EMEM;
     /* A partition count the caller asked for gets the reference's layout
@@ -614,14 +621,22 @@ static int plan_create(int n, long long nnz, int ku, int kl, int is_complex, int
      * partitions, since a long last partition's chain would set the time
      * (with many small partitions the remainder can be a hundred blocks). */
     const int nreg = n / p, rem = partitions > 0 ? 0 : n % p;
-    for (int i = 0; i < p; i++) {
-        const int s = i * nreg + (i < rem ? i : rem), e = i + 1 < p ? (i + 1) * nreg + (i + 1 < rem ? i + 1 : rem) : n;
-        const int m = (e - s) / sub, more = (e - s) % sub;
-        for (int j = 0; j < sub; j++) ps[(size_t)i * sub + j] = s + j * m + (j < more ? j : more);
+    int rc = SPK_EMEM;
+    /* (the pieces' interfaces take memory: where they do not fit, p partitions still may) */
+    for (int q = sub; q > 0 && rc == SPK_EMEM; q = q > 1 ? 1 : 0) {
+        for (int i = 0; i < p; i++) {
+            const int s = i * nreg + (i < rem ? i : rem),
+                      e = i + 1 < p ? (i + 1) * nreg + (i + 1 < rem ? i + 1 : rem) : n;
+            const int m = (e - s) / q, more = (e - s) % q;
+            for (int j = 0; j < q; j++) ps[(size_t)i * q + j] = s + j * m + (j < more ? j : more);
+        }
+        ps[(size_t)p * q] = n;
+        rc = spk_plan_build(n, nnz, ku, kl, KB, is_complex, mode, p * q, ps, nrhs_max, stream, stream_alloc, out);
     }
-    ps[(size_t)p * sub] = n;
-    const int rc = spk_plan_build(n, nnz, ku, kl, KB, is_complex, mode, p * sub, ps, nrhs_max, stream, stream_alloc, out);
-    if (rc == SPK_OK) (*out)->p_user = p;
+    if (rc == SPK_OK) {
+        (*out)->p_user = p;
+        (*out)->sub = sub;
+    }
     free(ps);
     return rc;
 }
@@ -632,7 +647,7 @@ size_t spk_solve_footprint(int n, long long nnz, int k, int nrhs, int is_complex
     const int KB = spk_choose_block(k < 1 ? 1 : k);
     if (!KB || n <= 0) return 0;
     int p = choose_partitions(n, KB, partitions, is_complex);
-    const int nreg = n / p, sub = subdivision(n, KB, partitions, p);
+    const int nreg = n / p, sub = subdivision(n, KB, partitions, 1, p);
     /* blocks of m rows in `pieces` balanced pieces: m % pieces of them hold one row more */
 #define PIECES(m, pieces)                                                                                       \
     (((m) % (pieces)) * (((m) / (pieces) + 1 + KB - 1) / KB) +                                                  \
@@ -673,14 +688,21 @@ size_t spk_solve_footprint(int n, long long nnz, int k, int nrhs, int is_complex
     return b;
 }
 
-static int plan_matches(const spk_plan *P, int n, int ku, int kl, int is_complex, int mode, int partitions, int nrhs)
+/* the plan's partitions are those of this request */
+static int same_partitions(const spk_plan *P, int partitions, int split)
+{
+    return P->p_user == choose_partitions(P->n, P->KB, partitions, P->is_complex) &&
+           P->sub == subdivision(P->n, P->KB, partitions, split, P->p_user);
+}
+
+static int plan_matches(const spk_plan *P, int n, int ku, int kl, int is_complex, int mode, int partitions, int split,
+                        int nrhs)
 {
     if (!P) return 0;
     const int k = ku > kl ? ku : kl;
     const int KB = spk_choose_block(k < 1 ? 1 : k);
     return P->n == n && P->KB == KB && P->is_complex == is_complex && P->mode == mode &&
-           P->p_user == choose_partitions(n, KB, partitions, is_complex) &&
-           P->p == P->p_user * subdivision(n, KB, partitions, P->p_user) && nrhs <= P->nrhs_max;
+           same_partitions(P, partitions, split) && nrhs <= P->nrhs_max;
 }
 
 /* ------------------------------------------------------------------ */
@@ -857,8 +879,7 @@ static int run_device(spike_context_t c, int n, long long nnz, int nrhs, const i
      * call fall back to analysis, a new plan and a second factorization. */
     spk_plan *Q = c->plan;
     if (Q && Q->n == n && Q->nnz == nnz && Q->is_complex == is_complex && Q->mode == c->mode &&
-        Q->p_user == choose_partitions(n, Q->KB, c->partitions, is_complex) &&
-        Q->p == Q->p_user * subdivision(n, Q->KB, c->partitions, Q->p_user) && chunk0 <= Q->nrhs_max) {
+        same_partitions(Q, c->partitions, c->split) && chunk0 <= Q->nrhs_max) {
         unsigned e[4];
         Q->twist = Q->twist_cap && c->twist;
         Q->red_fp64 = c->red_fp64 && Q->KB <= 64;
@@ -899,11 +920,11 @@ static int run_device(spike_context_t c, int n, long long nnz, int nrhs, const i
     TRY(arc);
     if (info[2]) return SPK_ECSR;
     const int chunk = nrhs < RHS_CHUNK ? nrhs : RHS_CHUNK;
-    if (!plan_matches(c->plan, n, info[0], info[1], is_complex, c->mode, c->partitions, chunk)) {
+    if (!plan_matches(c->plan, n, info[0], info[1], is_complex, c->mode, c->partitions, c->split, chunk)) {
         spk_plan_destroy(c->plan);
         c->plan = NULL;
-        TRY(plan_create(n, nnz, info[0], info[1], is_complex, c->mode, c->partitions, chunk, c->stream, c->stream_alloc,
-                        &c->plan));
+        TRY(plan_create(n, nnz, info[0], info[1], is_complex, c->mode, c->partitions, c->split, chunk, c->stream,
+                        c->stream_alloc, &c->plan));
     }
     spk_plan *P = c->plan;
     P->nnz = nnz;
@@ -1081,9 +1102,7 @@ static int host_pipelined(spike_context_t c, int n, long long nnz, int nrhs, con
     spk_plan *Q = c->plan;
     const int chunk = nrhs < RHS_CHUNK ? nrhs : RHS_CHUNK;
     if (!Q || Q->n != n || Q->nnz != nnz || Q->is_complex != cplx || Q->mode != c->mode || !Q->twist_cap || !c->twist ||
-        Q->p_user != choose_partitions(n, Q->KB, c->partitions, cplx) ||
-        Q->p != Q->p_user * subdivision(n, Q->KB, c->partitions, Q->p_user) || chunk > Q->nrhs_max ||
-        Q->p < PIPE_RANGES ||
+        !same_partitions(Q, c->partitions, c->split) || chunk > Q->nrhs_max || Q->p < PIPE_RANGES ||
         Q->KB < 16 || Q->KB > 64 ||
         nnz < (8LL << 20) || c->timing)
         return SPK_EARG;
@@ -1420,8 +1439,8 @@ static Error_t factor_common(spike_context_t c, int cplx, const char *name, inte
     if (rc == SPK_OK) rc = spk_analyze(n, nnz, f->d_rowptr, f->d_colind, c->d_scratch, info, c->stream, &l0);
     if (rc == SPK_OK && info[2]) rc = SPK_ECSR;
     if (rc == SPK_OK)
-        rc = plan_create(n, nnz, info[0], info[1], cplx, c->mode, c->partitions, RHS_CHUNK, c->stream, c->stream_alloc,
-                         &f->plan);
+        rc = plan_create(n, nnz, info[0], info[1], cplx, c->mode, c->partitions, c->split, RHS_CHUNK, c->stream,
+                         c->stream_alloc, &f->plan);
     if (rc == SPK_OK) {
         f->plan->launches = l0;
         f->plan->twist = f->plan->twist_cap && c->twist;

@@ -83,6 +83,7 @@ typedef struct spk_plan {
     /* problem */
     int n, nrhs_max, ku, kl, KB, p;
     int p_user; /* the partition count the caller sees: p, or what p subdivides (plan_create) */
+    int sub;    /* the pieces each of them was to be split into: p = p_user * sub, or p_user where memory was short */
     int is_complex, mode;
     long long nnz;
     /* schedule (host copies) */

@@ -34,7 +34,8 @@ typedef struct spike_factor_s *spike_factor_t;
 /* ---- options (spike_set_option) ---- */
 #define SPIKE_OPT_PRECISION 0      /* SPIKE_PRECISION_MIXED (default) or _FP64 */
 #define SPIKE_OPT_PARTITIONS 1     /* 0 = automatic (default), else p (partitions long enough to leave the GPU
-                                      idle are split further inside; p's boundaries stay partition boundaries) */
+                                      idle are split further inside; p's boundaries stay partition boundaries;
+                                      SPIKE_OPT_SPLIT_PARTITIONS) */
 #define SPIKE_OPT_MAX_REFINE 2     /* correction sweeps after the first solve (default 3) */
 #define SPIKE_OPT_TOLERANCE 3      /* relative residual target (default 1e-12) */
 #define SPIKE_OPT_REDUCED_REFINE 4 /* FP64 refinement sweeps on the reduced system (default 2 mixed, 1 FP64) */
@@ -52,6 +53,10 @@ typedef struct spike_factor_s *spike_factor_t;
                                       check that the CSR is the full band while its values travel, so
                                       the column indices stay on the host (default 8; 0 = always copy
                                       them) */
+
+#define SPIKE_OPT_SPLIT_PARTITIONS 10 /* 0 = a requested partition count is exactly the count of partitions (and
+                                      of the reduced system's blocks, less one); 1 = long ones may be split
+                                      (default 1) */
 
 #define SPIKE_PRECISION_MIXED 0 /* FP32 / complex64 factors, FP64 residual + update + reduced solve */
 #define SPIKE_PRECISION_FP64 1  /* FP64 / complex128 everywhere */
