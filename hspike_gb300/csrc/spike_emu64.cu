@@ -25,48 +25,6 @@ template <int KB> struct EmuSmem {
     static constexpr size_t red = head + E::PLANES + 4 * tile;
 };
 
-// KB rows of KB doubles, `ld` apart in shared memory, by bulk copies on bar; warp 0 calls
-template <int KB> __device__ __forceinline__ void bulk_rows(double *s, int ld, const double *g, uint64_t *bar)
-{
-    const int lane = threadIdx.x & 31;
-    if (lane == 0) {
-        fence_proxy_async();
-        mbar_arrive_expect_tx(bar, KB * KB * 8);
-    }
-    __syncwarp();
-    for (int r = lane; r < KB; r += 32) bulk_g2s(s + (size_t)r * ld, g + (size_t)r * KB, KB * 8, bar);
-}
-
-// one shared buffer that bulk copies fill: all threads call issue() after a
-// barrier that ends its last use, and wait()
-template <int KB> struct EmuBar {
-    uint64_t *bar;
-    unsigned phase;
-    bool inflight;
-    __device__ __forceinline__ void issue(double *s, int ld, const double *g)
-    {
-        if (threadIdx.x < 32) bulk_rows<KB>(s, ld, g, bar);
-        inflight = true;
-    }
-    // false in every thread when the copy never landed (a barrier inside)
-    __device__ __forceinline__ bool wait()
-    {
-        const bool ok = mbar_wait(bar, phase);
-        phase ^= 1u;
-        inflight = false;
-        return !__syncthreads_or(!ok);
-    }
-    __device__ __forceinline__ void drain()
-    {
-        if (inflight) mbar_wait(bar, phase);
-    }
-};
-
-__device__ __forceinline__ void emu_timeout(unsigned *err)
-{
-    if (threadIdx.x == 0) atomicOr(err, SPK_DEV_ERR_TIMEOUT);
-}
-
 // L_J = F G, S_J = D - L E, G_J = S^{-1}, z_J = -L z_{J-1} (z_0 = C^)
 template <int KB>
 __global__ void __launch_bounds__(Emu<KB>::NT, 1)
@@ -98,13 +56,13 @@ __global__ void __launch_bounds__(Emu<KB>::NT, 1)
         double *gLj = gL + tb + (size_t)J * TS, *gGj = gG + tb + (size_t)J * TS;
         if (J > 0) {
             const double *gGp = gGj - TS;
-            if (!bF.wait()) return emu_timeout(err); // (and every thread built G's planes)
+            if (!bF.wait()) return emu_leave(err, bD, bF, bE); // (and every thread built G's planes)
             // L_J; A(J, J-1) is upper triangular (KB >= kl)
             em.product({sF, 1, LDC, gGp, 1, KB, nullptr, 0, 0, sL, LD, 1, gLj, 1, KB, 1, false});
-            if (!bE.wait()) return emu_timeout(err); // E_{J-1}; L_J is complete
+            if (!bE.wait()) return emu_leave(err, bD, bF, bE); // E_{J-1}; L_J is complete
             if (J + 1 < N) bF.issue(sF, LDC, gTp + (size_t)(J + 1) * 3 * TS + TS);
             em.template build<KB>(sE, LD, 1, KB);
-            if (!bD.wait()) return emu_timeout(err);
+            if (!bD.wait()) return emu_leave(err, bD, bF, bE);
             // S_J = D_J - L_J E_{J-1}; A(J-1, J) is lower triangular
             em.product({sL, LD, 1, sE, LD, 1, sS, LD, 1, sS, LD, 1, nullptr, 0, 0, 3, true});
             __syncthreads();
@@ -117,7 +75,7 @@ __global__ void __launch_bounds__(Emu<KB>::NT, 1)
                 __syncthreads();
             }
         } else if (!bD.wait()) {
-            return emu_timeout(err);
+            return emu_leave(err, bD, bF, bE);
         }
         ok = em.inverse_tile(sS, sL, sE) && ok; // (L_J and E_{J-1} have been used)
         if (J + 1 < N) bE.issue(sE, LD, gTp + (size_t)J * 3 * TS + 2 * TS);
@@ -194,7 +152,7 @@ __global__ void __launch_bounds__(Emu<KB>::NT, 1)
         double *xj = gX + tb + (size_t)J * TS;
         const bool hasZ = !isV || J == J0 || (o > 0 && J == J0 + 1);
         if (J < N - 1) {
-            if (!bE.wait()) return emu_timeout(err); // (and X_{J+1}'s planes are built)
+            if (!bE.wait()) return emu_leave(err, bG, bE); // (and X_{J+1}'s planes are built)
             // T = Z_J - E_J X_{J+1}; A(J, J+1) is lower triangular
             em.product({sE, 1, LDC, sX, LD, 1, hasZ ? zj : nullptr, KB, 1, sT, LD, 1, nullptr, 0, 0, 2, true});
             __syncthreads();
@@ -204,7 +162,7 @@ __global__ void __launch_bounds__(Emu<KB>::NT, 1)
         }
         if (J > 0) bE.issue(sE, LDC, gE + tb + (size_t)(J - 1) * TS);
         em.template build<KB>(sT, LD, 1, KB);
-        if (!bG.wait()) return emu_timeout(err);
+        if (!bG.wait()) return emu_leave(err, bG, bE);
         em.product({sG, 1, LDC, sT, LD, 1, nullptr, 0, 0, sX, LD, 1, xj, 1, KB, 0, false});
         __syncthreads();
         if (J > 0) {

@@ -477,3 +477,49 @@ template <int KB> struct Emu {
         return ok;
     }
 };
+
+// KB rows of KB doubles, `ld` apart in shared memory, by bulk copies on bar; warp 0 calls
+template <int KB> __device__ __forceinline__ void bulk_rows(double *s, int ld, const double *g, uint64_t *bar)
+{
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) {
+        fence_proxy_async();
+        mbar_arrive_expect_tx(bar, KB * KB * 8);
+    }
+    __syncwarp();
+    for (int r = lane; r < KB; r += 32) bulk_g2s(s + (size_t)r * ld, g + (size_t)r * KB, KB * 8, bar);
+}
+
+// one shared buffer that bulk copies fill: all threads call issue() after a
+// barrier that ends its last use, and wait()
+template <int KB> struct EmuBar {
+    uint64_t *bar;
+    unsigned phase;
+    bool inflight;
+    __device__ __forceinline__ void issue(double *s, int ld, const double *g)
+    {
+        if (threadIdx.x < 32) bulk_rows<KB>(s, ld, g, bar);
+        inflight = true;
+    }
+    // false in every thread when the copy has not landed in time (a barrier
+    // inside): it still counts as in flight
+    __device__ __forceinline__ bool wait()
+    {
+        if (__syncthreads_or(!mbar_wait(bar, phase))) return false;
+        phase ^= 1u;
+        inflight = false;
+        return true;
+    }
+    __device__ __forceinline__ void drain()
+    {
+        if (inflight) mbar_wait(bar, phase);
+    }
+};
+
+// a wait has run out: say so, and give every copy still in flight the time of
+// one more wait, since the block's shared memory is another's once it leaves
+template <class... Bar> __device__ __forceinline__ void emu_leave(unsigned *err, Bar &...b)
+{
+    if (threadIdx.x == 0) atomicOr(err, SPK_DEV_ERR_TIMEOUT);
+    (b.drain(), ...);
+}

@@ -127,6 +127,7 @@ template <class T, int KB, int NRC, int NT> struct RsSeg {
         const bool ok = mbar_wait(bar, 0);
         if (__syncthreads_or(!ok)) {
             if (threadIdx.x == 0) atomicOr(A.err, SPK_DEV_ERR_TIMEOUT);
+            mbar_wait(bar, 0); // once more: the shared memory is another block's after this one
             return false;
         }
         return true;

@@ -148,14 +148,15 @@ __global__ void __launch_bounds__(32 * NW * KS, 2)
             if (lane == 0 && e) atomicMax(&ec[uhk[u] >> 16], (int)e);
         }
         const bool landed = mbar_wait(bar, phase);
-        phase ^= 1u;
         if (__syncthreads_or(!landed)) { // no norm: the solve must not take this for converged
             if (tid == 0) {
                 atomicOr(err, SPK_DEV_ERR_TIMEOUT);
                 norms[0] = __longlong_as_double(0x7ff8000000000000ll);
             }
+            mbar_wait(bar, phase); // once more: the shared memory is another block's after this one
             return;
         }
+        phase ^= 1u;
         const bool inner = R0 >= kl && R0 + ROWS <= n - ku; // rows of ku + kl + 1 entries each
         const int wid = ku + kl + 1;
         for (int i = warp; i < ROWS; i += WARPS) {

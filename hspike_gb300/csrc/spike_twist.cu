@@ -909,6 +909,7 @@ __global__ void __launch_bounds__(TwVW::NT, 8)
         }
         if (__syncthreads_or(tmo)) { // every thread has used the piece (and X's rows)
             if (threadIdx.x == 0) atomicOr(err, SPK_DEV_ERR_TIMEOUT);
+            mbar_wait(bars + (s & 1), (unsigned)(s >> 1) & 1u); // copies in flight: once more each
             if (s + 1 < 8 * cnt) mbar_wait(bars + ((s + 1) & 1), (unsigned)((s + 1) >> 1) & 1u);
             return;
         }
