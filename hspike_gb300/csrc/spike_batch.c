@@ -194,7 +194,7 @@ static int group_build_plan(struct spike_batch_s *B, bgroup *G, int KB, int rpp)
         if (B->ku[G->members[j]] > ku) ku = B->ku[G->members[j]];
         if (B->kl[G->members[j]] > kl) kl = B->kl[G->members[j]];
     }
-    int rc = spk_plan_build((int)G->rows, G->nnz, ku, kl, KB, 0, B->ctx->mode, (int)p, ps, G->nrhs, G->stream, 0,
+    int rc = spk_plan_build((int)G->rows, G->nnz, ku, kl, KB, 0, B->ctx->mode, (int)p, ps, G->nrhs, 0, G->stream, 0,
                             &G->P);
     if (rc == SPK_OK) G->P->twist = G->P->twist_cap && B->ctx->twist;
     if (rc == SPK_OK) G->P->red_fp64 = B->ctx->red_fp64 && G->P->KB <= 64;

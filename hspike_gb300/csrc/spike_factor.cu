@@ -1231,7 +1231,7 @@ __global__ void k_tips(const int *__restrict__ part_start, const int *__restrict
 template <class T, class S, int KB> int launch_tips(spk_plan *P, cudaStream_t st)
 {
     using H = typename HighOf<T>::type;
-    const bool r = KB <= 16 || P->want_r;
+    const bool r = spk_keeps_r(P);
     k_tips<T, S, KB><<<dim3(P->n_iface, KB >= 32 ? 4 : 1, KB >= 32 ? KB / 32 : 1), KB <= 4 ? 64 : 256, 0, st>>>(
         P->d_part_start, P->d_blk_off, P->p, (const T *)P->d_V, (const T *)P->d_W, (S *)P->d_crP, (S *)P->d_crQ,
         (S *)P->d_crX, (S *)P->d_crY, r ? (H *)P->d_RP : nullptr, r ? (H *)P->d_RQ : nullptr,

@@ -396,7 +396,7 @@ void spk_plan_destroy(spk_plan *P)
     spk_phase_destroy(P);
     void *ptrs[] = {P->d_part_start, P->d_blk_off, P->d_blk_part, P->d_L, P->d_G, P->d_E, P->d_V, P->d_W,
                     P->d_Bhat, P->d_T, P->d_RP, P->d_RQ, P->d_RX, P->d_RY, P->d_crP, P->d_crQ, P->d_crX, P->d_crY,
-                    P->d_crM, P->d_crg, P->d_z, P->d_y, P->d_g, P->d_u, P->d_rr, P->d_du, P->d_err, P->d_norms};
+                    P->d_crM, P->d_crg, P->d_z, P->d_y, P->d_g, P->d_u, P->d_rr, P->d_err, P->d_norms};
     for (size_t i = 0; i < sizeof ptrs / sizeof ptrs[0]; i++) spk_free_on(ptrs[i], P->astream);
     free(P->part_start);
     free(P->blk_off);
@@ -471,7 +471,6 @@ int spk_plan_reduced_build(int p, int KB, int is_complex, int mode, int nrhs_max
     PA(P->d_g, hs * nif * 2 * KB * nrhs_max);
     PA(P->d_u, hs * nif * 2 * KB * nrhs_max);
     PA(P->d_rr, hs * nif * 2 * KB * nrhs_max);
-    PA(P->d_du, hs * nif * 2 * KB * nrhs_max);
     PA(P->d_err, sizeof(unsigned) * 4);
 #undef PA
     if (rc != SPK_OK) {
@@ -483,7 +482,7 @@ int spk_plan_reduced_build(int p, int KB, int is_complex, int mode, int nrhs_max
 }
 
 int spk_plan_build(int n, long long nnz, int ku, int kl, int KB, int is_complex, int mode, int p,
-                   const int *part_start, int nrhs_max, void *stream, int stream_alloc, spk_plan **out)
+                   const int *part_start, int nrhs_max, int want_r, void *stream, int stream_alloc, spk_plan **out)
 {
     *out = NULL;
     if (!KB || spk_factor_smem(KB, is_complex, mode) == 0) return SPK_EBAND;
@@ -501,6 +500,7 @@ int spk_plan_build(int n, long long nnz, int ku, int kl, int KB, int is_complex,
     P->p = p;
     P->p_user = p;
     P->sub = 1;
+    P->want_r = want_r;
     P->n_iface = p - 1;
     P->part_start = (int *)malloc(sizeof(int) * (p + 1));
     P->blk_off = (int *)malloc(sizeof(int) * (p + 1));
@@ -567,10 +567,12 @@ int spk_plan_build(int n, long long nnz, int ku, int kl, int KB, int is_complex,
     PA(P->d_V, fs * TS * P->total_blocks);
     PA(P->d_Bhat, fs * TS * p);
     PA(P->d_T, fs * TS * 3 * P->total_blocks);
-    PA(P->d_RP, hs * TS * nif);
-    PA(P->d_RQ, hs * TS * nif);
-    PA(P->d_RX, hs * TS * nif);
-    PA(P->d_RY, hs * TS * nif);
+    if (spk_keeps_r(P)) {
+        PA(P->d_RP, hs * TS * nif);
+        PA(P->d_RQ, hs * TS * nif);
+        PA(P->d_RX, hs * TS * nif);
+        PA(P->d_RY, hs * TS * nif);
+    }
     PA(P->d_crP, hs * TS * tiles); /* FP64 scalars: the reduced system may run in FP64 (red_fp64) */
     PA(P->d_crQ, hs * TS * tiles);
     PA(P->d_crX, hs * TS * tiles);
@@ -582,7 +584,6 @@ int spk_plan_build(int n, long long nnz, int ku, int kl, int KB, int is_complex,
     PA(P->d_g, hs * nif * 2 * KB * nrhs_max);
     PA(P->d_u, hs * nif * 2 * KB * nrhs_max);
     PA(P->d_rr, hs * nif * 2 * KB * nrhs_max);
-    PA(P->d_du, hs * nif * 2 * KB * nrhs_max);
     PA(P->d_err, sizeof(unsigned) * 4);
     PA(P->d_norms, sizeof(double) * 2 * nrhs_max);
 #undef PA
@@ -631,7 +632,7 @@ static int plan_create(int n, long long nnz, int ku, int kl, int is_complex, int
             for (int j = 0; j < q; j++) ps[(size_t)i * q + j] = s + j * m + (j < more ? j : more);
         }
         ps[(size_t)p * q] = n;
-        rc = spk_plan_build(n, nnz, ku, kl, KB, is_complex, mode, p * q, ps, nrhs_max, stream, stream_alloc, out);
+        rc = spk_plan_build(n, nnz, ku, kl, KB, is_complex, mode, p * q, ps, nrhs_max, 0, stream, stream_alloc, out);
     }
     if (rc == SPK_OK) {
         (*out)->p_user = p;
@@ -677,11 +678,11 @@ size_t spk_solve_footprint(int n, long long nnz, int k, int nrhs, int is_complex
     size_t b = 0;
     b += sizeof(int) * (2 * (size_t)(p + 1) + (size_t)blocks);
     b += fs * TS * (size_t)blocks * 8 + fs * TS * p;            /* L G E W V + 3 band tiles, B^ */
-    b += hs * TS * (size_t)nif * 4;                               /* RP RQ RX RY */
+    if (KB <= SPK_R_MAX_KB) b += hs * TS * (size_t)nif * 4;       /* RP RQ RX RY */
     b += hs * TS * (size_t)tiles * 4 + hs * TS * 4 * (size_t)mtiles; /* cyclic reduction (FP64 scalars) */
     b += hs * 2 * (size_t)tiles * 2 * KB * chunk;                 /* reduced RHS work */
     b += fs * 2 * (size_t)blocks * KB * chunk;                    /* z, y */
-    b += hs * (size_t)nif * 2 * KB * chunk * 4;                   /* g u rr du */
+    b += hs * (size_t)nif * 2 * KB * chunk * 3;                   /* g u rr */
     b += 16 + sizeof(double) * 2 * chunk;
     /* staging of a host-array solve: CSR, b, x, r */
     b += sizeof(int) * ((size_t)n + 1 + (size_t)nnz) + hs * (size_t)nnz + hs * (size_t)n * (2 * nrhs + chunk);
@@ -1666,10 +1667,12 @@ Error_t spike_dsolve_device_noalloc(integer_t n, integer_t nnz, integer_t nrhs, 
     CV(P.d_V, fs * TS * P.total_blocks);
     CV(P.d_Bhat, fs * TS * p);
     CV(P.d_T, fs * TS * 3 * P.total_blocks);
-    CV(P.d_RP, hs * TS * nif);
-    CV(P.d_RQ, hs * TS * nif);
-    CV(P.d_RX, hs * TS * nif);
-    CV(P.d_RY, hs * TS * nif);
+    if (spk_keeps_r(&P)) {
+        CV(P.d_RP, hs * TS * nif);
+        CV(P.d_RQ, hs * TS * nif);
+        CV(P.d_RX, hs * TS * nif);
+        CV(P.d_RY, hs * TS * nif);
+    }
     CV(P.d_crP, fs * TS * tiles);
     CV(P.d_crQ, fs * TS * tiles);
     CV(P.d_crX, fs * TS * tiles);
@@ -1681,7 +1684,6 @@ Error_t spike_dsolve_device_noalloc(integer_t n, integer_t nnz, integer_t nrhs, 
     CV(P.d_g, hs * nif * 2 * KB * nr);
     CV(P.d_u, hs * nif * 2 * KB * nr);
     CV(P.d_rr, hs * nif * 2 * KB * nr);
-    CV(P.d_du, hs * nif * 2 * KB * nr);
     CV(P.d_err, sizeof(unsigned) * 4);
     CV(P.d_norms, sizeof(double) * 2 * nr);
     void *d_r = carve(&cv, hs * (size_t)n * nr);

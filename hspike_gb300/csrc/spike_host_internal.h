@@ -63,7 +63,7 @@ SPK_INTERNAL int spk_choose_block(int k);
 /* A plan for an explicit schedule: tile size KB, p partitions starting at
  * part_start[0..p] (part_start[p] = n).  Allocates the device workspace. */
 SPK_INTERNAL int spk_plan_build(int n, long long nnz, int ku, int kl, int KB, int is_complex, int mode, int p,
-                                const int *part_start, int nrhs_max, void *stream, int stream_alloc,
+                                const int *part_start, int nrhs_max, int want_r, void *stream, int stream_alloc,
                                 spk_plan **out);
 /* The reduced system of p partitions (p - 1 interfaces, tile size KB) alone:
  * the arrays of spk_reduced_factor / spk_reduced_solve, nothing else. */

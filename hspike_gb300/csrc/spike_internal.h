@@ -118,7 +118,7 @@ typedef struct spk_plan {
     void *d_L, *d_G, *d_E, *d_V, *d_W; /* V, W tiles are column-major */
     void *d_Bhat;                      /* [p][KB][KB] */
     void *d_T;                         /* [total_blocks][3][KB][KB]: D, F^T, E per block (row-major) */
-    /* reduced system: level-0 quadrant blocks in FP64 (or complex128) */
+    /* reduced system: level-0 quadrant blocks in FP64 (or complex128), where something reads them (spk_keeps_r) */
     void *d_RP, *d_RQ, *d_RX, *d_RY; /* [n_iface][KB][KB] */
     int want_r;     /* d_RP .. d_RY are read from outside (a sharded solve's records): keep them at every tile size */
     int red_direct; /* the tips wrote the cyclic reduction's level-0 blocks themselves (else they come from d_RP ..) */
@@ -134,7 +134,6 @@ typedef struct spk_plan {
     /* right-hand-side work (per solve) */
     void *d_z, *d_y;       /* factor precision, NP x nrhs_max */
     void *d_g, *d_u, *d_rr; /* FP64 reduced RHS, solution, reduced residual: n_iface*2KB x nrhs_max */
-    void *d_du;            /* FP64 reduced correction */
     unsigned int *d_err;   /* device error word */
     /* batch groups only (NULL otherwise): per-system table and the system
      * of each partition; CSR, b and x are then read through the table */
@@ -153,6 +152,13 @@ typedef struct spk_plan {
     double phase_ms[SPK_NPHASES];
     long long phase_calls[SPK_NPHASES];
 } spk_plan;
+
+/* The level-0 blocks are kept in FP64 for tiles up to SPK_R_MAX_KB rows, whose
+ * residual on R reads them (larger tiles' reads the cyclic reduction's own), and
+ * for the records of a sharded solve. */
+#define SPK_R_MAX_KB 16
+static inline int spk_keeps_r(const spk_plan *P) { return P->KB <= SPK_R_MAX_KB || P->want_r; }
+
 
 /* phase timing: begin/end record events on the stream; collect (after a
  * stream synchronize) adds the elapsed times to phase_ms / phase_calls */

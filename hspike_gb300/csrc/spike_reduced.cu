@@ -634,15 +634,19 @@ template <int KB> int run_red_factor_c(spk_plan *P, cudaStream_t st)
     static bool attr = false;
     if (!attr) {
         const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        if (cudaFuncSetAttribute(k_cr_schur<KB, 32>, a, (int)C::SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_cr_quads<KB, 32>, a, (int)C::SMEM) != cudaSuccess ||
+        if (cudaFuncSetAttribute(k_cr_quads<KB, 32>, a, (int)C::SMEM) != cudaSuccess ||
             cudaFuncSetAttribute(k_cr_even_cols<KB, 32>, a, (int)C::SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_cr_schur<KB, FINE>, a, (int)C2::SMEM) != cudaSuccess ||
             cudaFuncSetAttribute(k_cr_quads<KB, FINE>, a, (int)C2::SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_cr_even_cols<KB, FINE>, a, (int)C2::SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_cr_schur_inv<KB>, a, (int)(2 * INV)) != cudaSuccess ||
-            cudaFuncSetAttribute(k_cr_inv<KB>, a, (int)INV) != cudaSuccess)
+            cudaFuncSetAttribute(k_cr_even_cols<KB, FINE>, a, (int)C2::SMEM) != cudaSuccess)
             return SPK_ECUDA;
+        if constexpr (KB <= 64) {
+            if (cudaFuncSetAttribute(k_cr_schur_inv<KB>, a, (int)(2 * INV)) != cudaSuccess) return SPK_ECUDA;
+        } else {
+            if (cudaFuncSetAttribute(k_cr_schur<KB, 32>, a, (int)C::SMEM) != cudaSuccess ||
+                cudaFuncSetAttribute(k_cr_schur<KB, FINE>, a, (int)C2::SMEM) != cudaSuccess ||
+                cudaFuncSetAttribute(k_cr_inv<KB>, a, (int)INV) != cudaSuccess)
+                return SPK_ECUDA;
+        }
         attr = true;
     }
     float *cP = (float *)P->d_crP, *cQ = (float *)P->d_crQ, *cX = (float *)P->d_crX, *cY = (float *)P->d_crY,

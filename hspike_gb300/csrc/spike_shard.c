@@ -231,10 +231,10 @@ static int shard_plans(shard_t *S, int KB)
     ps[0] = 0;
     for (int j = 0; j <= np; j++) ps[1 + j] = h + (int)(part_row(S->n, p, S->part0 + j) - S->row0);
     ps[pl] = nl;
-    int rc = spk_plan_build(nl, S->nnz_loc, KB, KB, KB, 0, c->mode, pl, ps, nr, c->stream, 0, &S->P);
+    /* (want_r: its interface blocks travel as FP64 records) */
+    int rc = spk_plan_build(nl, S->nnz_loc, KB, KB, KB, 0, c->mode, pl, ps, nr, 1, c->stream, 0, &S->P);
     free(ps);
     TRY(rc);
-    S->P->want_r = 1; /* its interface blocks travel as FP64 records */
     const size_t vb = sizeof(double) * (size_t)nl * nr;
     TRY(spk_malloc((void **)&S->d_b, vb));
     TRY(spk_malloc((void **)&S->d_x, vb));

@@ -65,6 +65,24 @@ int main(void)
     /* not for four either */
     cap = 1000;
     CHECK(plan_create(n, 0, k, k, 0, SPK_PLAIN, p, 1, 1, NULL, 0, &P) == SPK_EMEM && !P && used == 0);
+    cap = (size_t)-1;
+    /* what a plan holds is what the admission estimate says, at every tile size;
+     * FP64 copies of the reduced system's blocks only where they are read */
+    const int ks[] = {1, 3, 8, 16, 17, 40, 64, 100};
+    for (int i = 0; i < 8; i++)
+        for (int mode = SPK_MIXED; mode <= SPK_PLAIN; mode++)
+            for (int parts = 0; parts <= 5; parts += 5) {
+                const int nn = 30011, nr = 3;
+                CHECK(plan_create(nn, 0, ks[i], ks[i], 0, mode, parts, 1, nr, NULL, 0, &P) == SPK_OK);
+                const size_t staging = sizeof(int) * ((size_t)nn + 1) + 8 * (size_t)nn * 3 * nr;
+                CHECK(P->bytes == used);
+                CHECK(spk_solve_footprint(nn, 0, ks[i], nr, 0, mode, parts) == P->bytes + staging);
+                CHECK((P->d_RP != NULL) == (P->KB <= 16) && (P->d_RY != NULL) == (P->KB <= 16));
+                spk_plan_destroy(P);
+            }
+    CHECK(spk_plan_reduced_build(9, 64, 0, SPK_MIXED, 2, &P) == SPK_OK && P->d_RP && P->d_RY);
+    spk_plan_destroy(P);
+    CHECK(used == 0);
     /* the option itself */
     struct spike_context_s c = {.split = 1};
     double v = 0;

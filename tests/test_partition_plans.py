@@ -1,5 +1,6 @@
 """Requested partition counts: split inside by default, exactly p on request,
-and exactly p as well where the pieces do not fit the device's memory."""
+and exactly p as well where the pieces do not fit the device's memory; and what
+any plan holds against the estimate that requests are admitted by."""
 import os
 import subprocess
 
