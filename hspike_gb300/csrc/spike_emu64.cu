@@ -5,8 +5,8 @@
 // (spike_factor.cu) and k_cr_odd / k_cr_even (spike_reduced.cu), which the FP64
 // pipe bounds: 73 + 55 + 5 ms of the 139 ms of n = 2,000,000, k = 64 in plain
 // FP64, for 3 KB^3 multiply-adds per block and direction.  With digit products
-// the three take 30 + 19 + 3 ms: a step's three products 27,000 clocks each, its
-// inverse 125,000.  One CTA of 256 threads fills an SM: the right operand's digit
+// the three take 35 + 16 + 3 ms: a step's three products 23,000 clocks each, its
+// inverse 134,000.  One CTA of 256 threads fills an SM: the right operand's digit
 // planes take 83 KB, three working tiles 111 KB, and the next block's coupling
 // tiles arrive by bulk copies in what is free.
 #include "spike_emu64.cuh"
@@ -19,7 +19,7 @@ template <int KB> struct EmuSmem {
     using E = Emu<KB>;
     static constexpr size_t tile = sizeof(double) * E::TILE;
     static constexpr size_t ctile = sizeof(double) * KB * E::LDC;
-    static constexpr size_t head = 64 + sizeof(int) * E::EC_INTS; // mbarriers, scales
+    static constexpr size_t head = 64 + E::AUX; // mbarriers, scales, lists
     static constexpr size_t fwd = head + E::PLANES + 3 * tile + ctile;
     static constexpr size_t bwd = head + E::PLANES + 2 * tile + 2 * ctile;
     static constexpr size_t red = head + E::PLANES + 4 * tile;
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(Emu<KB>::NT, 1)
         } else if (!bD.wait()) {
             return emu_leave(err, bD, bF, bE);
         }
-        ok = em.inverse_tile(sS, sL, sE) && ok; // (L_J and E_{J-1} have been used)
+        ok = em.inverse(sS, sL) && ok; // (L_J has been used)
         if (J + 1 < N) bE.issue(sE, LD, gTp + (size_t)J * 3 * TS + 2 * TS);
         for (int q = threadIdx.x; q < KB * KB; q += E::NT) { // column-major, 8 x 4 pieces per warp
             const int w = q >> 5, r = (w % (KB / 8)) * 8 + (q & 7), c = w / (KB / 8) * 4 + ((q >> 3) & 3);
@@ -202,12 +202,9 @@ __global__ void __launch_bounds__(Emu<KB>::NT, 1)
     __syncthreads();
     em.product({sQ, LD, 1, sP, LD, 1, sH, LD, 1, sH, LD, 1, nullptr, 0, 0, 0, true}); // S
     __syncthreads();
-    const bool ok = em.inverse_tile(sH, sX, sQ);
+    const bool ok = em.inverse(sH, sX);
     if (!ok) atomicOr(err, SPK_DEV_ERR_PIVOT);
-    for (int q = threadIdx.x; q < KB * KB; q += E::NT) {
-        Mj[3 * TS + q] = sH[q / KB * LD + q % KB];
-        sQ[q / KB * LD + q % KB] = Q[q]; // (the inverse's scratch)
-    }
+    for (int q = threadIdx.x; q < KB * KB; q += E::NT) Mj[3 * TS + q] = sH[q / KB * LD + q % KB];
     em.template build<KB>(sH, LD, 1, KB);
     __syncthreads();
     em.product({sP, LD, 1, sH, LD, 1, nullptr, 0, 0, Mj + TS, KB, 1, nullptr, 0, 0, 0, true}); // M01
