@@ -1415,7 +1415,7 @@ template <class T, int KB> int run_apply(spk_plan *P, const void *r, int nrhs, c
         rc = P->twist ? run_tw_apply<T, KB>(P, r, nrhs, st) : run_apply_1<T, KB>(P, r, nrhs, st);
     if (rc != SPK_OK) return rc;
     if (P->n_iface > 0) {
-        if (launch_dep(k_ytips<T, KB>, dim3(P->n_iface), 128, 0, 1, !P->d_sys, st, (const int *)P->d_part_start,
+        if (launch_dep(k_ytips<T, KB>, dim3(P->n_iface), 128, 0, 1, chained(P), st, (const int *)P->d_part_start,
                        (const int *)P->d_blk_off, (const T *)P->d_y, P->NP, nrhs, P->n_iface,
                        (typename HighOf<T>::type *)P->d_g) != SPK_OK)
             return SPK_ECUDA;
@@ -1432,14 +1432,13 @@ template <class T, int KB> int run_retrieve(spk_plan *P, void *x, int nrhs, int 
     // unknowns per spike convert their own where they are few: n = 1,000, k = 2
     // saves a launch of 3 us, n = 4,000,000, k = 3, complex, four columns would pay 330 us
     // a pass.  Each launch may start while the one before runs out (that and the
-    // narrowing: 172 -> 150 us for the small solve), but not in a batch, where
-    // waiting CTAs take another group's place (512 systems: 8.2 ms against 8.0).
+    // narrowing: 172 -> 150 us for the small solve).
     constexpr bool SAME = std::is_same<T, H>::value;
     const bool own = KB <= 4 && P->NP * nrhs <= 1 << 16, narrow = !SAME && !own;
     T *ut = SAME ? (T *)P->d_u : (T *)P->d_crg;
     const long long cnt = (long long)(P->n_iface > 0 ? P->n_iface : 1) * 2 * KB * nrhs;
     if (narrow && P->n_iface > 0) {
-        if (launch_dep(k_u_narrow<T>, dim3((unsigned)std::min<long long>((cnt + 255) / 256, 4096)), 256, 0, 1, !P->d_sys, st,
+        if (launch_dep(k_u_narrow<T>, dim3((unsigned)std::min<long long>((cnt + 255) / 256, 4096)), 256, 0, 1, chained(P), st,
                        (const H *)P->d_u, ut, cnt) != SPK_OK)
             return SPK_ECUDA;
         P->launches++;
@@ -1453,7 +1452,7 @@ template <class T, int KB> int run_retrieve(spk_plan *P, void *x, int nrhs, int 
             const long long tot = P->NP * nrhs;
             const int grid = (int)std::min<long long>((tot + 255) / 256, (long long)cap);
             auto go = [&](auto kern, auto *u) {
-                return launch_dep(kern, dim3(grid), 256, 0, 1, !P->d_sys, st, (const int *)P->d_part_start,
+                return launch_dep(kern, dim3(grid), 256, 0, 1, chained(P), st, (const int *)P->d_part_start,
                                   (const int *)P->d_blk_off, P->p, (const int *)P->d_blk_part, (const T *)P->d_V,
                                   (const T *)P->d_W, (const T *)P->d_y, u, P->NP, P->n_iface, P->n, nrhs, (H *)x,
                                   accumulate, (const spk_sysref *)P->d_sys, (const int *)P->d_part_sys);
@@ -1463,7 +1462,7 @@ template <class T, int KB> int run_retrieve(spk_plan *P, void *x, int nrhs, int 
         } else {
             const long long tot = P->NP * ((nrhs + RET_HC - 1) / RET_HC);
             const int grid = (int)std::min<long long>((tot + 255) / 256, (long long)cap);
-            if (launch_dep(k_retrieve_rows<T, KB>, dim3(grid), 256, 0, 1, !P->d_sys, st, (const int *)P->d_part_start,
+            if (launch_dep(k_retrieve_rows<T, KB>, dim3(grid), 256, 0, 1, chained(P), st, (const int *)P->d_part_start,
                            (const int *)P->d_blk_off, P->p, (const int *)P->d_blk_part, (const T *)P->d_V,
                            (const T *)P->d_W, (const T *)P->d_y, (const T *)ut, P->NP, P->n_iface, P->n, nrhs, (H *)x,
                            accumulate, (const spk_sysref *)P->d_sys, (const int *)P->d_part_sys) != SPK_OK)
@@ -1481,7 +1480,7 @@ template <class T, int KB> int run_retrieve(spk_plan *P, void *x, int nrhs, int 
                     return SPK_ECUDA;
                 attr = true;
             }
-            return launch_dep(k_retrieve<T, KB, HC>, dim3(P->total_blocks), 256, C::SMEM, 1, !P->d_sys, st,
+            return launch_dep(k_retrieve<T, KB, HC>, dim3(P->total_blocks), 256, C::SMEM, 1, chained(P), st,
                               (const int *)P->d_part_start, (const int *)P->d_blk_off, P->p, (const int *)P->d_blk_part,
                               (const T *)P->d_V, (const T *)P->d_W, (const T *)P->d_y, (const T *)ut, P->NP, P->n_iface,
                               P->n, nrhs, (H *)x, accumulate, (const spk_sysref *)P->d_sys, (const int *)P->d_part_sys);

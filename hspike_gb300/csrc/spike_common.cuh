@@ -1624,9 +1624,14 @@ __device__ __forceinline__ char *smem_align(char *p)
 // (programmatic dependent launch): it does what does not depend on the
 // predecessor and then waits for it (dep_wait).  The first kernel of a chain is
 // launched plainly, and every kernel of the chain waits, so what was complete
-// before the chain is complete for all of it.
+// before the chain is complete for all of it.  Not in a batch, whose groups run
+// side by side: CTAs that wait there take another group's place (the reduced
+// systems of 512 systems 7.03 ms against 6.92 without, of 64 1.99 against 1.95).
+// A server's slots, which have a GPU's room between them, measure the same both ways.
 __device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+static inline bool chained(const spk_plan *P) { return !P->d_sys; }
 
 template <class Kern, class... Args>
 static int launch_dep(Kern k, dim3 grid, int nt, size_t smem, int cluster, bool dep, cudaStream_t st, Args... args)

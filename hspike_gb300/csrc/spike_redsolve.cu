@@ -437,6 +437,7 @@ template <class T, int KB, int NRC> int run_red_solve_s(spk_plan *P, int nrhs, i
     auto bytes = [&](int n, int levels, bool top) { return rs_bytes<T>(n, levels, KB, NRC, top); };
     int tier[RS_MAXL + 1], nt;
     const int lt = rs_schedule(lv, SMEM, bytes, tier, nt);
+    const bool chain = chained(P);
     bool dep = false; // the first kernel of the solve starts after everything before it
     for (int it = 0; it < (lt == 0 ? 1 : iters); it++) {
         int rc = SPK_OK;
@@ -445,12 +446,12 @@ template <class T, int KB, int NRC> int run_red_solve_s(spk_plan *P, int nrhs, i
             const int segs = (lv.cnt[l0] + (1 << s) - 1) >> s;
             rc = launch_dep(k_rs_fwd<T, KB, NRC>, dim3(segs, hy), RS_NT, bytes((1 << s) + 1, s, false), 1, dep, st, A,
                             lv, l0, l1, (int)(it > 0));
-            dep = true;
+            dep = chain;
         }
         if (rc == SPK_OK)
             rc = launch_dep(k_rs_top<T, KB, NRC>, dim3(1, hy), RS_TOP_NT, bytes(lv.cnt[lt], L - lt, true), 1, dep, st,
                             A, lv, lt, iters);
-        dep = true;
+        dep = chain;
         for (int q = nt - 1; q >= 0 && rc == SPK_OK; q--) {
             const int l0 = tier[q], l1 = tier[q + 1], s = l1 - l0;
             const int segs = (lv.cnt[l0] + (1 << s) - 1) >> s;
@@ -884,13 +885,14 @@ template <class T, int KB, int NRC> int run_red_solve_q(spk_plan *P, int nrhs, i
     const T *cX = (const T *)P->d_crX, *cY = (const T *)P->d_crY, *cM = (const T *)P->d_crM;
     const int L = P->cr_levels;
     const unsigned hy = (nrhs + NRC - 1) / NRC;
+    const bool chain = chained(P); // (every kernel but the first)
     for (int it = 0; it < iters; it++) {
         const H *res = it == 0 ? (const H *)P->d_g : (const H *)P->d_rr;
         auto in = [&](int l) { return l == 0 ? (const void *)res : (const void *)cgv; };
         auto ld = [&](int l) { return l == 0 ? NR : stride; };
         for (int l = 0; l < L; l++) {
             const int cnt = P->cr_count[l];
-            if (launch_dep(k_crq_fwd<T, KB, NRC>, dim3((cnt + 1) / 2 * Q::CS, hy), QNT, 0, Q::CS, it + l > 0, st,
+            if (launch_dep(k_crq_fwd<T, KB, NRC>, dim3((cnt + 1) / 2 * Q::CS, hy), QNT, 0, Q::CS, chain && it + l > 0, st,
                                cX + (size_t)P->cr_off[l] * TS, cY + (size_t)P->cr_off[l] * TS,
                                cM + (size_t)P->cr_moff[l] * 4 * TS, cnt, in(l), (int)(l == 0), ld(l),
                                (long long)P->cr_off[l], cgv, stride, (long long)P->cr_off[l + 1], nrhs) != SPK_OK)
@@ -898,7 +900,7 @@ template <class T, int KB, int NRC> int run_red_solve_q(spk_plan *P, int nrhs, i
         }
         for (int l = L; l >= 0; l--) { // level L: the top block
             const int cnt = P->cr_count[l], nodd = l == L ? 1 : cnt / 2;
-            if (launch_dep(k_crq_bwd<T, KB, NRC>, dim3(nodd * Q::CS, hy), QNT, 0, Q::CS, it + L > 0, st,
+            if (launch_dep(k_crq_bwd<T, KB, NRC>, dim3(nodd * Q::CS, hy), QNT, 0, Q::CS, chain && it + L > 0, st,
                                cX + (size_t)P->cr_off[l] * TS, cY + (size_t)P->cr_off[l] * TS,
                                cM + (size_t)P->cr_moff[l] * 4 * TS, cnt, in(l), (int)(l == 0), ld(l),
                                (long long)P->cr_off[l], cu, stride, l, (H *)P->d_u, NR, (int)(it == 0), nrhs,
@@ -914,9 +916,9 @@ template <class T, int KB, int NRC> int run_red_solve_q(spk_plan *P, int nrhs, i
             if constexpr (std::is_same<T, float>::value && NRC > 1) {
                 using S = RedSl<KB>;
                 rc = launch_dep(k_red_resid_sl<KB>, dim3(P->n_iface * S::CPI, (nrhs + S::NC - 1) / S::NC), S::NT, 0, 1,
-                                true, st, (const T *)P->d_crP, (const T *)P->d_crQ, cX, cY, (const H *)P->d_g,
+                                chain, st, (const T *)P->d_crP, (const T *)P->d_crQ, cX, cY, (const H *)P->d_g,
                                 (const H *)P->d_u, (H *)P->d_rr, P->n_iface, nrhs);
-            } else if (launch_dep(k_red_resid<T, KB, RC>, dim3(P->n_iface * Q::CS, (nrhs + RC - 1) / RC), QNT, 0, 1, true, st,
+            } else if (launch_dep(k_red_resid<T, KB, RC>, dim3(P->n_iface * Q::CS, (nrhs + RC - 1) / RC), QNT, 0, 1, chain, st,
                            (const T *)P->d_crP, (const T *)P->d_crQ, cX, cY, (const H *)P->d_g, (const H *)P->d_u, (H *)P->d_rr, P->n_iface, nrhs) != SPK_OK)
                 rc = SPK_ECUDA;
             if (rc != SPK_OK) return rc;

@@ -612,7 +612,7 @@ template <class T, int KB> int run_red_factor_s(spk_plan *P, cudaStream_t st)
     auto run = [&](auto kern, int grid, int nthr, size_t smem, int l0, int l1, int top) {
         const int rc = launch_dep(kern, dim3(grid), nthr, smem, 1, dep, st, (T *)P->d_crP, (T *)P->d_crQ,
                                   (T *)P->d_crX, (T *)P->d_crY, (T *)P->d_crM, lv, l0, l1, top, P->d_err);
-        dep = true;
+        dep = chained(P);
         P->launches++;
         return rc;
     };
@@ -655,7 +655,7 @@ template <int KB> int run_red_factor_c(spk_plan *P, cudaStream_t st)
     int rc = SPK_OK;
     auto run = [&](auto kern, dim3 grid, size_t smem, auto... args) {
         if (rc == SPK_OK) rc = launch_dep(kern, grid, C::NT, smem, 1, dep, st, args...);
-        dep = true;
+        dep = chained(P);
         P->launches++;
     };
     auto odd = [&](const float *p, const float *q, int first, int stride, int count, float *M) {
