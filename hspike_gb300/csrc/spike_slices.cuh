@@ -1,4 +1,4 @@
-// spike_slices.cuh -- FP64 dot products on the tensor cores, exactly.
+// spike_slices.cuh -- FP64 dot products on the tensor cores, by exact products of digits.
 //
 // GB300 retires 2 FP64 multiply-adds per clock and SM, its tensor cores about
 // a thousand FP16 ones.  An FP64 value that shares a power-of-two scale with
@@ -11,15 +11,22 @@
 //
 // takes one m16n8k16 product per digit pair with the FP32 accumulator of each
 // s exact as long as it holds at most SL_FLUSH k steps: 8 pairs x 2^14 x 128
-// <= 2^24 at s = 7.  The pairs with s >= 8 are left out: together they stay
-// below 2^-58 of the two scales' product, while an FP64 sum rounds at 2^-53 of
-// the partial sums (the splitting is Ozaki, Ogita, Oishi, Rump's, Numer.
-// Algorithms 59, 2012, with the digits taken by bytes).
+// <= 2^24 at s = 7 (the splitting is Ozaki, Ogita, Oishi, Rump's, Numer.
+// Algorithms 59, 2012, with the digits taken by bytes).  The pairs with s >= 8 are
+// left out: per term at most 7.03 x 2^14 x 256^6, 2^-57.2 of the two scales'
+// product, and the bits of values far below their scale that shift out of the
+// digits, at most 2^-59.  A sum of K terms can miss K times that, 2^-51 of the
+// scales' product at K = 64 and 2^-49 at 257, where every digit is near its
+// extreme and of one sign; unrelated digits miss sqrt(K) 2^-60, 2^-57 and 2^-56.
 //
-// What the scales could lose -- values far below the largest of their row or
-// column -- is watched by one more product, of |x| and |y| as powers of two:
-// where sum |x||y| is below SL_GUARD of the scales' product the caller forms
-// that result in FP64 as before.
+// That is measured by the scales, an FP64 sum's error by the terms it adds.  So
+// the scales' reach is watched by one more product, of |x| and |y| as powers of
+// two rounded down: where sum |x||y| is below SL_GUARD of the scales' product the
+// caller forms that result in FP64 as before.  Above it a result misses at most
+// 2^6 times the above of its terms' magnitudes, 2^-50 for unrelated digits (an FP64
+// chain of K terms: up to K 2^-53), and where the terms come near the scales, as in
+// the rows of a dominant band, less than the chain's roundings (K = 129, terms of
+// one magnitude: rms 2.6e-16 against 2.2e-14).
 #pragma once
 #include <cuda_fp16.h>
 
@@ -27,7 +34,7 @@
 
 constexpr int SL_D = 8;              // digits
 constexpr int SL_FLUSH = 8;          // k steps (of 16) an FP32 accumulator holds exactly
-constexpr float SL_GUARD = 0.015625f; // 2^-6 (the magnitudes are rounded down to powers of two)
+constexpr float SL_GUARD = 0.015625f; // 2^-6
 
 // biased exponent of |v| (0 for zero and subnormals, 0x7ff for inf and NaN)
 __device__ __forceinline__ int sl_exp(double v) { return (int)(((unsigned)__double2hiint(v) >> 20) & 0x7ffu); }
