@@ -47,7 +47,7 @@ struct RtGeom {
         const size_t p = (size_t)(SL_D + 1) * nc * ldx * sizeof(__half), e = (size_t)ks * rows * nc * 20;
         return ((p > e ? p : e) + 15) & ~(size_t)15;
     }
-    __host__ __device__ size_t bytes() const { return 16 + 2 * 16 * 8 + 64 + 256 + planes() + (size_t)cap * 8; }
+    __host__ __device__ size_t bytes() const { return 16 + (2 + 8) * 16 * 8 + 64 + 256 + planes() + (size_t)cap * 8; }
 };
 
 // entries of a full band before row r (modulo 2^32: the true value fits an int)
@@ -55,6 +55,66 @@ __device__ __forceinline__ int band_off(int r, int n, int ku, int kl)
 {
     const unsigned m = (unsigned)min(r, kl), q = (unsigned)max(0, r - (n - ku));
     return (int)((unsigned)r * (unsigned)(ku + kl + 1) - (m * (unsigned)kl - m * (m - 1u) / 2u) - q * (q + 1u) / 2u);
+}
+
+// The results of a tile of rows from R0 on without digits, from the values
+// sv[band_off(row) ..]: four rows per warp at a time and all of a row's columns
+// together, eight lanes to a row, so that a value of A is read once and a result
+// costs 68 clocks of the FP64 pipe at k = 64 (86 in k_residual, 160 one by one).
+// Squared norms go into sw, a warp's own sixteen values.  (A call: the digits' loop
+// needs its registers.)
+template <int ROWS, int WARPS>
+__device__ __noinline__ void in_fp64(int R0, const double *sv, int n, int ku, int kl,
+                                     const double *__restrict__ x, const double *__restrict__ b, double *r, int nc,
+                                     int want_b, double *sw)
+{
+    constexpr int NC = RT_NC;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h = lane & 7;
+    double qr = 0.0, qb = 0.0; // squared norms of column h
+    for (int rg = warp * 4; rg < ROWS && R0 + rg < n; rg += WARPS * 4) {
+        const int row = R0 + rg + (lane >> 3), rl = min(row, n - 1), first = max(0, rl - kl);
+        const int len = row < n ? min(n - 1, row + ku) - first + 1 : 0;
+        const double *av = sv + band_off(rl, n, ku, kl), *xc = x + first;
+        const bool mine = row < n && h < nc;
+        const double bv = mine ? b[(size_t)h * n + row] : 0.0;
+        double f[NC];
+#pragma unroll
+        for (int c = 0; c < NC; c++) f[c] = 0.0;
+        for (int q = h; q < ku + kl + 1; q += 8) {
+            const bool on = q < len;
+            const double v = on ? av[q] : 0.0;
+#pragma unroll
+            for (int c = 0; c < NC; c++)
+                if (c < nc) f[c] = fma(v, on ? xc[(size_t)c * n + q] : 0.0, f[c]);
+        }
+        __syncwarp();
+        // column c's sum ends at lane c of the eight
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            const bool up = (h & o) != 0;
+#pragma unroll
+            for (int e = 0; e < o; e++) {
+                const double send = up ? f[e] : f[e + o];
+                f[e] = (up ? f[e + o] : f[e]) + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+        if (mine) {
+            const double rv = bv - f[0];
+            r[(size_t)h * n + row] = rv;
+            qr = fma(rv, rv, qr);
+            if (want_b) qb = fma(bv, bv, qb);
+        }
+    }
+#pragma unroll
+    for (int o = 8; o < 32; o *= 2) {
+        qr += __shfl_xor_sync(0xffffffffu, qr, o);
+        qb += __shfl_xor_sync(0xffffffffu, qb, o);
+    }
+    if (lane < 8) {
+        sw[warp * 16 + h] += qr;
+        sw[warp * 16 + 8 + h] += qb;
+    }
 }
 
 // NW groups of 16 rows, KS warps per group (each every KS-th k step, at most
@@ -72,7 +132,8 @@ __global__ void __launch_bounds__(32 * NW * KS, 2)
     extern __shared__ __align__(16) char sm[];
     uint64_t *bar = (uint64_t *)sm;
     double *sr = (double *)(sm + 16), *sb = sr + 16;  // squared norms of r and b per column
-    int *ec = (int *)(sb + 16), *er = ec + 16;        // scale exponents of the columns and rows
+    double *sw = sb + 16;                             // and, by warp, those of tiles without digits
+    int *ec = (int *)(sw + 8 * 16), *er = ec + 16; // scale exponents of the columns and rows
     char *pl = (char *)(er + 64);
     unsigned short *px = (unsigned short *)pl;        // [digit][column][ldx]; plane SL_D: magnitudes
     long long *xh = (long long *)pl, *xl = xh + KS * ROWS * NC; // partial sums, [ks][column][row]
@@ -81,7 +142,7 @@ __global__ void __launch_bounds__(32 * NW * KS, 2)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int wr = warp % NW, wk = warp / NW; // this warp's rows and k steps
-    if (tid < 32) sr[tid] = 0.0;              // sr, sb
+    for (int q = tid; q < 10 * 16; q += NTH) sr[q] = 0.0; // sr, sb, sw
     if (tid == 0) {
         mbar_init(bar, 1);
         mbar_init_fence();
@@ -129,6 +190,7 @@ __global__ void __launch_bounds__(32 * NW * KS, 2)
     double nr[OPT], nb[OPT];
 #pragma unroll
     for (int i = 0; i < OPT; i++) nr[i] = nb[i] = 0.0;
+    int skip = 0; // tiles yet to be formed without trying the digits
     if (tid == 0) fetch(blockIdx.x);
     window(blockIdx.x);
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -157,6 +219,14 @@ __global__ void __launch_bounds__(32 * NW * KS, 2)
             return;
         }
         phase ^= 1u;
+        if (skip > 0) {
+            skip--;
+            in_fp64<ROWS, WARPS>(R0, sa - e0, n, ku, kl, x, b, r, nc, want_b, sw);
+            __syncthreads(); // every value has been used
+            if (tid == 0) fetch(tile + gridDim.x);
+            window(tile + gridDim.x);
+            continue;
+        }
         const bool inner = R0 >= kl && R0 + ROWS <= n - ku; // rows of ku + kl + 1 entries each
         const int wid = ku + kl + 1;
         for (int i = warp; i < ROWS; i += WARPS) {
@@ -243,6 +313,7 @@ __global__ void __launch_bounds__(32 * NW * KS, 2)
         window(tile + gridDim.x); // lands while the results are formed
         __syncthreads();
         // ---- r = b - A x, a row of one column per thread
+        bool many = false;
 #pragma unroll
         for (int i = 0; i < OPT; i++) { // (whole warps: one column each, the same in every tile)
             const int o = tid + i * NTH, h = o / ROWS, rw = o - h * ROWS, row = R0 + rw;
@@ -261,7 +332,8 @@ __global__ void __launch_bounds__(32 * NW * KS, 2)
             const bool redo = live && !(E < 0x7ff && (Ec == 0 || (E >= 64 && Ec >= 64 && Ec < 0x7ff && mg >= SL_GUARD &&
                                                                  sc > -900 && sc < 850)));
             double ax = redo || Ec == 0 ? 0.0 : sl_round(hi, lo, sc);
-            // the few results outside the scales' reach, one by one in FP64
+            // the results outside the scales' reach, one by one in FP64
+            many = many || redo;
             for (unsigned todo = __ballot_sync(0xffffffffu, redo); todo; todo &= todo - 1) {
                 const int src = __ffs(todo) - 1, rr = __shfl_sync(0xffffffffu, row, src);
                 const int t0 = band_off(rr, n, ku, kl), len = band_off(rr + 1, n, ku, kl) - t0;
@@ -278,7 +350,13 @@ __global__ void __launch_bounds__(32 * NW * KS, 2)
                 if (want_b) nb[i] = fma(bv, bv, nb[i]);
             }
         }
-        __syncthreads(); // the partial sums may be overwritten by the next planes
+        // (The partial sums may be overwritten by the next planes.)  Where many results
+        // were formed in FP64 -- a solution that falls off between its sources -- what
+        // follows looks alike, and fifteen tiles go without trying the digits.  n = 400,000,
+        // two residuals, a source every 4 k rows: k = 64, 16 columns 8.47 -> 3.98 ms
+        // (k_residual 3.80), k = 24, 4 columns 1.46 -> 0.65 (0.45); n = 200,000, k = 100, 8
+        // columns 1.97 -> 1.46 (1.55).  U[-1,1] solutions pay 1.5 % for the count.
+        if (__syncthreads_count(many) > NTH / 4) skip = 15;
     }
 #pragma unroll
     for (int i = 0; i < OPT; i++) {
@@ -295,8 +373,13 @@ __global__ void __launch_bounds__(32 * NW * KS, 2)
     }
     __syncthreads();
     if (tid < nc) {
-        atomicAdd(&norms[tid], sr[tid]);
-        if (want_b) atomicAdd(&bnorms[tid], sb[tid]);
+        double qr = sr[tid], qb = sb[tid];
+        for (int w = 0; w < WARPS; w++) {
+            qr += sw[w * 16 + tid];
+            qb += sw[w * 16 + 8 + tid];
+        }
+        atomicAdd(&norms[tid], qr);
+        if (want_b) atomicAdd(&bnorms[tid], qb);
     }
 }
 
