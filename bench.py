@@ -39,10 +39,11 @@ WORKLOAD = (f"large-band real SPIKE: n={N:,} kl=ku={K_BAND} partitions={P} nrhs=
 
 # DRAM bytes (read + write) per row block of each kernel family, from one ncu
 # capture of this workload at full size (n = 2,000,000, 31,490 row blocks;
-# factor_fwd = k_tw_lu 79,741 + k_tw_sweep 30,961); rhs_sweeps from a capture
-# of `bench.py --n 600000 --partitions 300` (same 64-row tiles and partition
-# length).  Traffic per launch = this x the launch's row blocks.
-TRAFFIC_PER_BLOCK = {"factor_fwd": 110_702, "factor_bwd": 111_898, "band_tiles": 162_757, "rhs_sweeps": 48_796}
+# factor_fwd = k_tw_lu 79,690 + k_tw_sweep 30,953, factor_bwd = k_tw_bwd_vw);
+# rhs_sweeps from a capture of `bench.py --n 600000 --partitions 300` (same
+# 64-row tiles and partition length).  Traffic per launch = this x the launch's
+# row blocks.
+TRAFFIC_PER_BLOCK = {"factor_fwd": 110_643, "factor_bwd": 80_106, "band_tiles": 162_871, "rhs_sweeps": 48_796}
 
 
 def row_blocks(n, p, kb):
